@@ -1,0 +1,71 @@
+"""Grouped aggregation in shared-memory cells and limb sums: group counts at
+the edges of the modes, signs, row counts that fold the cells midway."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from oracle import oracle
+from ultraprecise_b200 import abi, codec, runtime
+from ultraprecise_b200 import expr as E
+
+pytestmark = pytest.mark.gpu
+
+AGGS = [(abi.UP_AGG_SUM, 0), (abi.UP_AGG_AVG, 1), (abi.UP_AGG_COUNT, 1)]
+
+
+def _raw(t):
+    return bytes(t.cpu().numpy().tobytes())
+
+
+# slots: 512 at p=18 (13 cells per group), 256 at p=38; register modes below 9 groups
+@pytest.mark.parametrize("p", [5, 18, 38])
+@pytest.mark.parametrize("groups,rows", [(1, 1), (8, 3000), (9, 30_011), (16, 4097), (17, 5000), (256, 20_000),
+                                         (257, 20_000), (511, 10_000), (513, 10_000), (2049, 40_001)])
+def test_group_counts_at_the_mode_edges(p, groups, rows):
+    a, b = E.col(0), E.col(1)
+    q = runtime.compile_query([a * b, a - b], AGGS, [E.ColType(p, 2)] * 2)
+    cols = [runtime.gen_digits(rows, p, 7 + k) for k in range(2)]
+    g = torch.Generator(device="cuda").manual_seed(groups)
+    # skewed ids, the largest id present
+    u = torch.rand(rows, device="cuda", generator=g)
+    gid = (u ** 4 * groups).to(torch.int32).clamp_(max=groups - 1)
+    gid[rows // 2] = groups - 1
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = q.launch([runtime.DeviceColumn(t, p, 2) for t in cols], gid, groups, err=err)
+    assert int(err.item()) == 0
+    exp = oracle.query(q.built, q.aggs, [_raw(t) for t in cols], _raw(gid), rows, groups, threads=8)
+    for k, (o, e) in enumerate(zip(outs, exp)):
+        assert _raw(o) == e, f"aggregate {k}"
+
+
+@pytest.mark.parametrize("groups", [12, 100_000])
+def test_cells_fold_midway(groups):
+    """More rows per CTA than the cells stay exact for (32768): values of one
+    sign and full pieces, sums checked as int64."""
+    rows, p = 24_000_000, 9
+    q = runtime.compile_query([E.col(0)], [(abi.UP_AGG_SUM, 0), (abi.UP_AGG_COUNT, 0)], [E.ColType(p, 0)])
+    v = torch.full((rows,), 0x3FFFFFF, dtype=torch.int64, device="cuda")  # 67108863: low piece 65535
+    v -= torch.arange(rows, device="cuda") % 3
+    raw = v.to(torch.int32).view(torch.uint8)
+    assert codec.compact_bytes(p) == 4
+    g = torch.Generator(device="cuda").manual_seed(3)
+    gid = (torch.rand(rows, device="cuda", generator=g) ** 3 * groups).to(torch.int32).clamp_(max=groups - 1)
+    outs = q.launch([runtime.DeviceColumn(raw, p, 0)], gid, groups)
+    want = torch.zeros(groups, dtype=torch.int64, device="cuda").index_add_(0, gid.long(), v).cpu().numpy()
+    img = outs[0].cpu().numpy().reshape(groups, abi.UP_AGG_DECIMAL_BYTES)
+    got = img[:, 5:13].copy().view(np.int64).reshape(-1)
+    assert np.array_equal(got, want) and not img[:, 13:].any() and not img[:, 1].any()
+    cnt = outs[1].cpu().numpy().view(np.int64)
+    assert np.array_equal(cnt, torch.bincount(gid.long(), minlength=groups).cpu().numpy())
+
+
+def test_group_ids_out_of_range_are_flagged():
+    rows, groups, p = 5000, 600, 18
+    q = runtime.compile_query([E.col(0) * E.col(1), E.col(0)], AGGS, [E.ColType(p, 2)] * 2)
+    cols = [runtime.gen_digits(rows, p, 3 + k) for k in range(2)]
+    gid = torch.arange(rows, device="cuda", dtype=torch.int32) % groups
+    gid[17], gid[18] = groups, -1
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    q.launch([runtime.DeviceColumn(t, p, 2) for t in cols], gid, groups, err=err)
+    assert int(err.item()) == 4  # UP_ROWERR_DOMAIN

@@ -423,6 +423,13 @@ size_t query_scratch_bytes(const GeneratedModule& g, int32_t n_groups) {
     return acc_bytes + (size_t)n_groups * 8u;
 }
 
+size_t query_scratch_bytes_max(const GeneratedModule& g, int32_t n_groups) {
+    const size_t limb = g.q_gs > 0 && n_groups > g.q_gs
+                            ? query_scratch_bytes(g, g.q_gs) + 32u + (size_t)n_groups * g.q_limb_words * 8u
+                            : 0u;
+    return std::max(limb, query_scratch_bytes(g, n_groups));
+}
+
 up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64_t rows, const int32_t* group_ids,
                           int32_t n_groups, void* const* outs, uint32_t* err_word, void* stream, bool spread,
                           const QueryKeys* keys, void* caller_scratch, size_t caller_scratch_bytes) {
@@ -447,8 +454,18 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
     if (sms <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t accw = (size_t)std::max(g.acc_words_per_group, 1);
-    const size_t acc_bytes = (((size_t)n_groups * accw * 4u) + 15u) & ~(size_t)15u;
-    const size_t need = query_scratch_bytes(g, n_groups);
+    size_t need = query_scratch_bytes(g, n_groups);
+    // More groups than cells: limb sums, which stay exact below 2^31 rows
+    // (every sum adds signed 32-bit limbs in 64 bits).  A count known on the
+    // host needs no accumulators beside them; a count on the device may turn
+    // out small enough for the cells, whose accumulators it keeps.
+    bool limbs = contig && g.q_staged && g.q_gs > 0 && n_groups > g.q_gs && rows < ((int64_t)1 << 31);
+    const int32_t acc_groups = limbs ? (device_count ? g.q_gs : 0) : n_groups;
+    const size_t limb_off = (query_scratch_bytes(g, acc_groups) + 31u) & ~(size_t)31u;
+    const size_t limb_need = limb_off + (size_t)n_groups * g.q_limb_words * 8u;
+    if (limbs && caller_scratch && limb_need > caller_scratch_bytes) limbs = false;
+    if (limbs) need = limb_need;
+    const size_t acc_bytes = (((size_t)(limbs ? acc_groups : n_groups) * accw * 4u) + 15u) & ~(size_t)15u;
     void* scratch = caller_scratch;
     if (caller_scratch) {
         if (need > caller_scratch_bytes)
@@ -463,6 +480,7 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
     a.gid = group_ids;
     a.acc = (uint32_t*)scratch;
     a.cnt = (unsigned long long*)((uint8_t*)scratch + acc_bytes);
+    a.lacc = limbs ? (long long*)((uint8_t*)scratch + limb_off) : nullptr;
     a.err = err_word;
     a.n_groups = device_count ? -n_groups : n_groups;
     a.vec_ok = vec_ok ? 1 : 0;
@@ -483,26 +501,29 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
             const bool reg_lo = g.q_gr_lo > 0 && n_groups <= g.q_gr_lo;
             const char* reg_name = keys ? "up_query_tile_rk" : "up_query_tile_r";
             const char* lo_name = keys ? "up_query_tile_rk_lo" : "up_query_tile_r_lo";
-            const char* name = reg_lo ? lo_name : reg ? reg_name : (n_groups <= g.q_gs) ? "up_query_tile_s"
-                                                                                        : "up_query_tile_g";
+            const char* name = reg_lo                             ? lo_name
+                               : reg                              ? reg_name
+                               : (n_groups <= g.q_gs || a.lacc) ? "up_query_tile_h"
+                                                                  : "up_query_tile_g";
             a.vec_ok = (vec_ok && keys_aligned) ? 1 : 0;
             const int64_t ntiles = (rows + g.q_tile_rows - 1) / g.q_tile_rows;
             auto launch_tile = [&](const char* kname) -> cudaError_t {
                 void* k = jit_kernel(*m->jm.ks, kname);
-                if (set_smem(k, g.q_smem) != UP_OK) return cudaErrorInvalidValue;  // layout kept within 48 KB
+                const int smem = kname[14] == 'h' ? g.q_smem_h : g.q_smem;  // up_query_tile_h
+                if (set_smem(k, smem) != UP_OK) return cudaErrorInvalidValue;
                 // the register and shared-memory modes merge once per CTA, so a
                 // spread launch keeps a bounded grid of several waves
-                const int64_t cap = (int64_t)sms * occupancy(k, g.block_threads, g.q_smem) * (spread ? 8 : 1);
+                const int64_t cap = (int64_t)sms * occupancy(k, g.block_threads, smem) * (spread ? 8 : 1);
                 return cudaLaunchKernel((const void*)k, dim3((unsigned)std::min<int64_t>(ntiles, cap)),
-                                        dim3(g.block_threads), args, (size_t)g.q_smem, s);
+                                        dim3(g.block_threads), args, (size_t)smem, s);
             };
             if (device_count) {
                 // the mode follows the count on the device: every applicable
                 // mode kernel is launched and all but one return at once
                 if (g.q_gr_lo > 0) e = launch_tile(lo_name);
                 if (e == cudaSuccess && g.q_gr > 0 && n_groups > g.q_gr_lo) e = launch_tile(reg_name);
-                if (e == cudaSuccess && (g.q_gr == 0 || n_groups > g.q_gr)) e = launch_tile("up_query_tile_s");
-                if (e == cudaSuccess && n_groups > g.q_gs) e = launch_tile("up_query_tile_g");
+                if (e == cudaSuccess && (g.q_gr == 0 || n_groups > g.q_gr)) e = launch_tile("up_query_tile_h");
+                if (e == cudaSuccess && n_groups > g.q_gs && !a.lacc) e = launch_tile("up_query_tile_g");
             } else {
                 e = launch_tile(name);
             }

@@ -1552,6 +1552,66 @@ UP_DI void atomic_acc_add(u32* acc, const u32 (&m)[N], u32 sign) {
     atomic_add_twos(acc, t);
 }
 
+// Cell accumulators: a group's running sum held as signed 16-bit pieces of
+// the magnitude, one 32-bit cell per piece in shared memory, S cells apart.
+// Adding a value is one atomic without a returned value and without a carry
+// per piece (a carry chain of atomics waits for every returned word); a cell
+// stays exact for kCellRows additions, after which the cells are folded into
+// the wide accumulators.
+constexpr int kCellRows = 32768;  // 32768 * 65535 < 2^31
+
+template <int S, int NP, int N>
+UP_DI void cells_add(int* cell, const u32 (&m)[N], u32 sign) {
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+        const int v = (int)((i & 1) ? m[i / 2] >> 16 : m[i / 2] & 0xffffu);
+        if (v) atomicAdd(cell + i * S, sign ? -v : v);
+    }
+}
+
+// limb l of a cell accumulator of NP pieces (signed)
+template <int S, int NP>
+UP_DI i64 cells_limb(const int* cell, int l) {
+    return (i64)cell[2 * l * S] + (2 * l + 1 < NP ? (i64)cell[(2 * l + 1) * S] * 65536 : 0ll);
+}
+
+// Slot of a group in a CTA's hash of S slots (tags: the slots' groups, -1
+// free): two candidate slots, the first comer keeps one; -1 when others hold
+// both.
+template <int S>
+UP_DI int cell_slot(int* tags, int g) {
+    const u32 h = ((u32)g * 0x9e3779b1u) >> 8;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int s = (int)((h & (u32)(S - 1)) ^ (u32)k);
+        int t = *(volatile int*)(tags + s);
+        if (t == -1) t = atomicCAS(tags + s, -1, g);
+        if (t == g || t == -1) return s;
+    }
+    return -1;
+}
+
+// Two's complement image over N limbs of a sum held as NL signed 64-bit limb
+// sums (each the sum of signed 32-bit limbs).
+template <int N, int NL>
+UP_DI void fold_limbs(u32 (&t)[N], const i64 (&l)[NL]) {
+    i64 c = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        c += i < NL ? l[i < NL ? i : 0] : 0ll;
+        t[i] = (u32)c;
+        c >>= 32;
+    }
+}
+
+// Add a value to limb sums in device memory: independent 64-bit reductions.
+template <int N>
+UP_DI void limb_sums_add(i64* acc, const u32 (&m)[N], u32 sign) {
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (m[i]) atomicAdd((u64*)(acc + i), (u64)(sign ? -(i64)m[i] : (i64)m[i]));
+}
+
 // The reference's nullable_type<Decimal> image of a SUM/AVG result
 // (decimal.hxx:130-140 plus the leading flag; kernel_segreduce.hxx:609-612):
 // [0] flag, [1] sign, [2] prec, [3] frac, [4] error, [5..133) v[32] LE.

@@ -97,8 +97,10 @@ struct GeneratedModule {
     int q_tile_rows = 0;          // rows per tile of the tile kernels
     int q_gr = 0;                 // up_query_tile_r handles n_groups <= q_gr
     int q_gr_lo = 0;              // up_query_tile_r_lo handles n_groups <= q_gr_lo (0: no such kernel)
-    int q_gs = 0;                 // up_query_tile_s handles n_groups <= q_gs
-    int q_smem = 0;               // dynamic shared memory of the tile kernels
+    int q_gs = 0;                 // slots of up_query_tile_h's cells: direct for n_groups <= q_gs, else hashed
+    int q_limb_words = 0;         // 64-bit words of one group's limb sums (hashed launches)
+    int q_smem = 0;               // dynamic shared memory of the _r and _g tile kernels
+    int q_smem_h = 0;             // of up_query_tile_h
     long work_per_row = 0;        // limb-product work + bytes per row (scheduling cost estimate)
     int threads_per_value = 1;    // threads cooperating on one value in the tile kernel
     // up_expr_multi (merged launches of several requests): rows per virtual
@@ -227,9 +229,12 @@ struct QueryKeys {
     // 131072) and may be at most `capacity`, which sizes the accumulators
     int capacity = 0;
 };
-// Scratch of a query launch for n_groups groups: the accumulators (16-byte
+// Scratch a query launch needs for n_groups groups: the accumulators (16-byte
 // padded) followed by one int64 count per group.
 size_t query_scratch_bytes(const upi::GeneratedModule& g, int32_t n_groups);
+// The most a launch allocates itself (the limb sums of a hashed launch may be
+// larger than its accumulators).
+size_t query_scratch_bytes_max(const upi::GeneratedModule& g, int32_t n_groups);
 // scratch: caller-provided device memory of scratch_bytes (at least
 // query_scratch_bytes, 16-byte aligned) used instead of a stream-ordered
 // allocation; the launch clears what it uses on `stream`.

@@ -38,7 +38,9 @@ struct UpArgs {
 // Query modules (up_query_*).  key_mode 0: group ids from gid[]; otherwise
 // the group is key_table[key] with key = key0[r] (1), key0[r] << 8 | key1[r]
 // (2), or key0[2r] << 8 | key0[2r+1] (3).  n_groups < 0: the count is read
-// from the key table on the device, -n_groups being the capacity.
+// from the key table on the device, -n_groups being the capacity.  lacc: the
+// limb sums of a launch whose groups outnumber its shared-memory cells (NULL:
+// its accumulators are in acc like the others').
 struct UpQArgs {
     UpKCol col[UP_MAX_COLS];
     unsigned char* out[UP_MAX_AGGS];
@@ -52,6 +54,7 @@ struct UpQArgs {
     const unsigned char* key0;
     const unsigned char* key1;
     const int* key_table;
+    long long* lacc;
     int key_mode;
 };
 
@@ -101,7 +104,7 @@ static_assert(sizeof(UpMultiReq) == 680, "UpMultiReq layout");
 static_assert(sizeof(UpMultiArgs) == 24, "UpMultiArgs layout");
 static_assert(sizeof(UpKCol) == 40, "UpKCol layout");
 static_assert(sizeof(UpArgs) == 672, "UpArgs layout");
-static_assert(sizeof(UpQArgs) == 848, "UpQArgs layout");
+static_assert(sizeof(UpQArgs) == 856, "UpQArgs layout");
 static_assert(sizeof(BTask) == 368, "BTask layout");
 static_assert(sizeof(BArgs) == 56, "BArgs layout");
 #endif

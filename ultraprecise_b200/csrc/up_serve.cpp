@@ -111,8 +111,7 @@ void size_request(Req& r, double heavy_work) {
             r.part_bytes.push_back((int64_t)r.n_groups * w);
             off += pad((int64_t)r.n_groups * w);
         }
-        const int64_t accw = std::max(g.acc_words_per_group, 1);
-        r.bytes = off + pad((int64_t)r.n_groups * accw * 4 + 16) + pad((int64_t)r.n_groups * 8);
+        r.bytes = off + pad((int64_t)query_scratch_bytes_max(g, r.n_groups) + 16);
     }
     r.out_bytes = off;
     r.heavy = heavy_work > 0 && (double)r.rows * (double)g.work_per_row > heavy_work;
