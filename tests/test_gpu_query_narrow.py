@@ -1,0 +1,86 @@
+"""The register kernels' narrow rows: columns at and around the narrow bounds,
+mixed with rows that need the general evaluation, against the oracle."""
+import random
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from oracle import oracle
+from ultraprecise_b200 import abi, codec, runtime
+from ultraprecise_b200 import expr as E
+
+pytestmark = pytest.mark.gpu
+
+
+def _raw(t):
+    return bytes(t.cpu().numpy().tobytes())
+
+
+def _column(rows, p, rng, wide):
+    """Values around every bound the narrow evaluation checks, of both signs."""
+    top = 10 ** p - 1
+    edges = [e for b in (20, 30, 31, 42, 47, 61, 62) for e in ((1 << b) - 1, 1 << b, (1 << b) + 1) if e <= top]
+    out = []
+    for _ in range(rows):
+        if rng.random() < wide:
+            m = rng.choice(edges + [top, 0]) if rng.random() < 0.5 else rng.randrange(top + 1)
+        else:
+            m = rng.randrange(min(top, 5_000_000) + 1)
+        out.append((rng.getrandbits(1), m))
+    return codec.encode(out, p)
+
+
+def _exprs(kind):
+    a, b, c = E.col(0), E.col(1), E.col(2)
+    if kind == "money":
+        d = a * (E.dec("1.00") - b)
+        return [a, d, d * (E.dec("1.00") + c), -b]
+    if kind == "sums":  # no product: columns up to 62 bits, three-word sums
+        return [a, a - b, (a + b) + E.dec("-3.5")]
+    return [a * a, a * b * c, E.lit(-7) * a]
+
+
+@pytest.mark.parametrize("kind", ["money", "sums", "products"])
+@pytest.mark.parametrize("p,groups,rows,wide", [(3, 1, 5, 0.0), (9, 4, 2051, 0.5), (12, 5, 4099, 0.02), (15, 7, 9001, 0.0),
+                                                (15, 4, 9001, 1.0), (18, 3, 3000, 0.3), (20, 8, 1027, 0.3),
+                                                (38, 6, 2500, 0.05)])
+def test_narrow_and_wide_rows(kind, p, groups, rows, wide):
+    rng = random.Random(p * 1000 + groups)
+    exprs = _exprs(kind)
+    aggs = [(abi.UP_AGG_SUM, i) for i in range(len(exprs))] + [(abi.UP_AGG_AVG, 0), (abi.UP_AGG_COUNT, 0)]
+    q = runtime.compile_query(exprs, aggs, [E.ColType(p, min(2, p - 1))] * 3)
+    raws = [_column(rows, p, rng, wide) for _ in range(3)]
+    cols = [runtime.DeviceColumn.from_host(r, p, min(2, p - 1)) for r in raws]
+    gid = torch.tensor([rng.randrange(groups) for _ in range(rows)], dtype=torch.int32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = q.launch(cols, gid, groups, err=err)
+    exp = oracle.query(q.built, q.aggs, raws, _raw(gid), rows, groups, threads=8)
+    assert int(err.item()) == 0
+    for k, (o, e) in enumerate(zip(outs, exp)):
+        assert _raw(o) == e, f"aggregate {k}"
+    # the same groups as one-byte, two-byte and 2 x one-byte keys
+    for keys, kb in (([gid.to(torch.uint8)], [1]), ([torch.stack([gid % 3, gid], 1).to(torch.uint8).reshape(-1)], [2]),
+                     ([(gid * 0 + 9).to(torch.uint8), gid.to(torch.uint8)], [1, 1])):
+        kid, n, _ = runtime.group_ids_from_keys(keys, kb)
+        table = torch.zeros(abi.UP_KEY_TABLE_ENTRIES, dtype=torch.int32, device="cuda")
+        runtime.group_table_from_keys_async(keys, kb, table)
+        got = q.launch_keys_async(cols, keys, kb, table, 64, err=err, rows=rows)
+        exp = oracle.query(q.built, q.aggs, raws, _raw(kid), rows, n, threads=8)
+        assert int(err.item()) == 0
+        for k, (o, e) in enumerate(zip(got, exp)):
+            assert _raw(o)[:len(e)] == e, f"keys {kb} aggregate {k}"
+
+
+def test_register_sums_over_many_tiles():
+    """More than 8192 tiles of 1024 rows for one CTA would take 2.4e9 rows; the
+    sums of 64M rows of the largest two-word values are checked as int64."""
+    rows, p = 1 << 26, 9
+    q = runtime.compile_query([E.col(0) * E.col(1)], [(abi.UP_AGG_SUM, 0), (abi.UP_AGG_COUNT, 0)], [E.ColType(p, 0)] * 2)
+    a = (torch.arange(rows, device="cuda", dtype=torch.int64) % 7 + 7_000_000).to(torch.int32)
+    b = torch.full((rows,), 9_000, dtype=torch.int32, device="cuda")
+    gid = (torch.arange(rows, device="cuda", dtype=torch.int32) % 3).to(torch.int32)
+    outs = q.launch([runtime.DeviceColumn(t.view(torch.uint8), p, 0) for t in (a, b)], gid, 3)
+    want = [int((a.long() * b.long())[gid == g].sum().item()) for g in range(3)]
+    got = [d["mag"] for d in codec.decode_agg(_raw(outs[0]), 3)]
+    assert got == want

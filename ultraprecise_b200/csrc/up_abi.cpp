@@ -506,16 +506,19 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
                                : (n_groups <= g.q_gs || a.lacc) ? "up_query_tile_h"
                                                                   : "up_query_tile_g";
             a.vec_ok = (vec_ok && keys_aligned) ? 1 : 0;
-            const int64_t ntiles = (rows + g.q_tile_rows - 1) / g.q_tile_rows;
             auto launch_tile = [&](const char* kname) -> cudaError_t {
                 void* k = jit_kernel(*m->jm.ks, kname);
-                const int smem = kname[14] == 'h' ? g.q_smem_h : g.q_smem;  // up_query_tile_h
+                const char mode = kname[14];  // up_query_tile_<mode>
+                const int smem = mode == 'h' ? g.q_smem_h : mode == 'r' ? g.q_smem_r : g.q_smem;
+                const int threads = mode == 'r' ? g.q_threads_r : g.block_threads;
+                const int tile_rows = mode == 'r' ? g.q_tile_rows_r : g.q_tile_rows;
+                const int64_t ntiles = (rows + tile_rows - 1) / tile_rows;
                 if (set_smem(k, smem) != UP_OK) return cudaErrorInvalidValue;
                 // the register and shared-memory modes merge once per CTA, so a
                 // spread launch keeps a bounded grid of several waves
-                const int64_t cap = (int64_t)sms * occupancy(k, g.block_threads, smem) * (spread ? 8 : 1);
+                const int64_t cap = (int64_t)sms * occupancy(k, threads, smem) * (spread ? 8 : 1);
                 return cudaLaunchKernel((const void*)k, dim3((unsigned)std::min<int64_t>(ntiles, cap)),
-                                        dim3(g.block_threads), args, (size_t)smem, s);
+                                        dim3(threads), args, (size_t)smem, s);
             };
             if (device_count) {
                 // the mode follows the count on the device: every applicable

@@ -1604,6 +1604,108 @@ UP_DI void fold_limbs(u32 (&t)[N], const i64 (&l)[NL]) {
     }
 }
 
+// A thread's register sum of one group: W words, two's complement.  Two words
+// hold 2^15 values below 2^47, three words 2^15 values below 2^63.
+template <int W>
+struct RSum;
+template <>
+struct RSum<2> {
+    i64 s;
+    UP_DI void clear() { s = 0; }
+    UP_DI void add(i64 v) { s += v; }
+    UP_DI u32 word(int i) const { return i ? (u32)((u64)s >> 32) : (u32)s; }
+    UP_DI void reduce_into(int* pieces, int lane);
+};
+template <>
+struct RSum<3> {
+    u32 w[3];
+    UP_DI void clear() { w[0] = w[1] = w[2] = 0u; }
+    UP_DI void add(i64 v) {
+        u64 c = (u64)w[0] + (u32)v;
+        w[0] = (u32)c;
+        c = (c >> 32) + w[1] + (u32)((u64)v >> 32);
+        w[1] = (u32)c;
+        w[2] += (u32)(c >> 32) + (u32)(v >> 63);
+    }
+    UP_DI u32 word(int i) const { return w[i]; }
+    UP_DI void reduce_into(int* pieces, int lane);
+};
+
+#ifndef UP_HOST_TEST
+// A warp's register sums into 16-bit pieces in shared memory (the top piece
+// signed): a CTA's 32 warps keep every piece below 2^26.
+template <int W>
+UP_DI void rsum_reduce(const RSum<W>& r, int* pieces, int lane) {
+#pragma unroll
+    for (int i = 0; i < 2 * W; i++) {
+        const u32 w = r.word(i / 2);
+        const int v = i == 2 * W - 1 ? (int)w >> 16 : (int)((i & 1) ? w >> 16 : w & 0xffffu);
+        const int t = __reduce_add_sync(0xffffffffu, v);
+        if (lane == 0 && t) atomicAdd(pieces + i, t);
+    }
+}
+UP_DI void RSum<2>::reduce_into(int* pieces, int lane) { rsum_reduce(*this, pieces, lane); }
+UP_DI void RSum<3>::reduce_into(int* pieces, int lane) { rsum_reduce(*this, pieces, lane); }
+
+// The bytes of four consecutive B-byte values (4*B bytes, a multiple of 4 in
+// a 16-byte aligned column tile): the widest loads B allows.  Thread strides
+// of an odd number of words, 8-byte or 16-byte units meet few bank conflicts.
+template <int B>
+UP_DI void ld_quad(u32 (&w)[B], const u8* p) {
+    if constexpr (B % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < B; i += 4) {
+            const uint4 v = *(const uint4*)(p + 4 * i);
+            w[i] = v.x;
+            w[i + 1] = v.y;
+            w[i + 2] = v.z;
+            w[i + 3] = v.w;
+        }
+    } else if constexpr (B % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < B; i += 2) {
+            const uint2 v = *(const uint2*)(p + 4 * i);
+            w[i] = v.x;
+            w[i + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < B; i++) w[i] = *(const u32*)(p + 4 * i);
+    }
+}
+#endif
+
+// 32 bits at byte offset o (a compile-time constant after unrolling)
+template <int W>
+UP_DI u32 word_at(const u32 (&w)[W], int o) {
+    return (o & 3) ? __funnelshift_r(at(w, o >> 2), at(w, (o >> 2) + 1), 8u * (u32)(o & 3)) : at(w, o >> 2);
+}
+
+// Value e of the four, as a signed integer, when its magnitude is below 2^C
+// (C <= 62); otherwise `bad` becomes nonzero.
+template <int B, int C>
+UP_DI i64 quad_value(const u32 (&w)[B], int e, u32& bad) {
+    constexpr int N = (B + 3) / 4, LAST = B - 4 * (N - 1);  // limbs, bytes of the last one
+    constexpr u32 MAG = LAST == 4 ? 0x7fffffffu : (1u << (8 * LAST - 1)) - 1u;
+    u32 m[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) m[i] = word_at(w, e * B + 4 * i);
+    const u32 neg = 0u - ((m[N - 1] >> (8 * LAST - 1)) & 1u);
+    m[N - 1] &= MAG;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        if (32 * i >= C) bad |= m[i];
+        else if (32 * i + 32 > C) bad |= m[i] >> (C - 32 * i);
+    }
+    if constexpr (C <= 31) {
+        return (i64)(int)((m[0] ^ neg) - neg);
+    } else {
+        const u64 v = (u64)m[0] | ((u64)at(m, 1) << 32);
+        const u64 n = (u64)(i64)(int)neg;
+        return (i64)((v ^ n) - n);
+    }
+}
+
 // Add a value to limb sums in device memory: independent 64-bit reductions.
 template <int N>
 UP_DI void limb_sums_add(i64* acc, const u32 (&m)[N], u32 sign) {

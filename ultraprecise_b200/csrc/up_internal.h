@@ -99,8 +99,10 @@ struct GeneratedModule {
     int q_gr_lo = 0;              // up_query_tile_r_lo handles n_groups <= q_gr_lo (0: no such kernel)
     int q_gs = 0;                 // slots of up_query_tile_h's cells: direct for n_groups <= q_gs, else hashed
     int q_limb_words = 0;         // 64-bit words of one group's limb sums (hashed launches)
-    int q_smem = 0;               // dynamic shared memory of the _r and _g tile kernels
+    int q_smem = 0;               // dynamic shared memory of up_query_tile_g
     int q_smem_h = 0;             // of up_query_tile_h
+    // the register kernels' shared memory, threads and rows per tile
+    int q_smem_r = 0, q_threads_r = 0, q_tile_rows_r = 0;
     long work_per_row = 0;        // limb-product work + bytes per row (scheduling cost estimate)
     int threads_per_value = 1;    // threads cooperating on one value in the tile kernel
     // up_expr_multi (merged launches of several requests): rows per virtual
