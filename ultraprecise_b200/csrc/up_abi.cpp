@@ -540,7 +540,8 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
     }
     if (e == cudaSuccess) {
         void* k = jit_kernel(*m->jm.ks, "up_query_fin");
-        e = cudaLaunchKernel((const void*)k, dim3((unsigned)((n_groups + 255) / 256)), dim3(256), args, 0, s);
+        e = cudaLaunchKernel((const void*)k, dim3((unsigned)((n_groups + kFinGroups - 1) / kFinGroups), (unsigned)g.n_aggs),
+                             dim3(kFinGroups), args, 0, s);
     }
     cudaError_t e2 = caller_scratch ? cudaSuccess : cudaFreeAsync(scratch, s);
     if (e != cudaSuccess) return cuda_fail(e, "query launch");

@@ -79,6 +79,7 @@ int rule_threads_per_value(const up_expr_node* nodes, const std::vector<NodeFact
 int coop_width_of(const up_expr_node* nodes, int n_nodes, int root, const up_col_type* cols, int n_cols);
 
 // ------------------------------------------------------------ code generation
+constexpr int kFinGroups = 128;  // groups per CTA of up_query_fin
 struct GeneratedModule {
     std::string source;
     std::vector<std::string> kernels;
