@@ -730,6 +730,74 @@ UP_DI void ld_compact_bytes(const u8* p, u32 (&m)[N], u32& sign) {
     m[TOPL] &= (TOPB == 31) ? 0x7fffffffu : ((1u << TOPB) - 1u);
 }
 
+// Word loads of a B-byte value anywhere in device memory whose column starts
+// on a 4-byte boundary: the words around the value's start hold bytes of the
+// same column, the last bytes are read one by one unless the value fills
+// their word, so nothing past the value is read.
+template <int B, int N>
+UP_DI void ld_compact_global(const u8* __restrict__ p, u32 (&m)[N], u32& sign) {
+    static_assert(N * 4 >= B, "limbs too few for the compact width");
+    constexpr int TOPL = (B - 1) / 4;
+    constexpr int TOPB = ((B - 1) % 4) * 8 + 7;
+    zero(m);
+    bool done = false;
+    if constexpr (B % 16 == 0) {
+        if (((unsigned long long)p & 15u) == 0u) {
+#pragma unroll
+            for (int i = 0; i < B / 16; i++) {
+                const uint4 v = ((const uint4*)p)[i];
+                m[4 * i] = v.x;
+                m[4 * i + 1] = v.y;
+                m[4 * i + 2] = v.z;
+                m[4 * i + 3] = v.w;
+            }
+            done = true;
+        }
+    } else if constexpr (B % 8 == 0) {
+        if (((unsigned long long)p & 7u) == 0u) {
+#pragma unroll
+            for (int i = 0; i < B / 8; i++) {
+                const uint2 v = ((const uint2*)p)[i];
+                m[2 * i] = v.x;
+                m[2 * i + 1] = v.y;
+            }
+            done = true;
+        }
+    }
+    if (!done) {
+        constexpr int W = (B + 3 + 3) / 4;  // words a value at any offset touches
+        const int off = (int)((unsigned long long)p & 3u), end = off + B;
+        const u8* q = p - off;
+        u32 x[W + 1];
+#pragma unroll
+        for (int i = 0; i < W; i++) {
+            if (4 * i + 4 <= B || 4 * i + 4 <= end) {
+                x[i] = ((const u32*)q)[i];
+            } else {
+                u32 v = 0u;
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                    if (4 * i + k < end) v |= (u32)q[4 * i + k] << (8 * k);
+                x[i] = v;
+            }
+        }
+        x[W] = 0u;
+#pragma unroll
+        for (int i = 0; i <= TOPL; i++) m[i] = __funnelshift_r(x[i], x[i + 1], 8u * (u32)off);
+    }
+    sign = (m[TOPL] >> TOPB) & 1u;
+    m[TOPL] &= (TOPB == 31) ? 0x7fffffffu : ((1u << TOPB) - 1u);
+}
+
+// A column value by how its memory may be read: 1 the words around it (a
+// padded tile), 2 whole words of the value's column only, 0 bytes.
+template <int B, int N>
+UP_DI void ld_compact(const u8* p, int words, u32 (&m)[N], u32& sign) {
+    if (words == 1) ld_compact_words<B, N>(p, m, sign);
+    else if (words == 2) ld_compact_global<B, N>(p, m, sign);
+    else ld_compact_bytes<B, N>(p, m, sign);
+}
+
 // Overflow test: any magnitude bit at or above 8*B-1 would be lost or would
 // collide with the sign bit.
 template <int B, int N>
@@ -1473,6 +1541,18 @@ UP_DI void tile_copy_out(u8* __restrict__ dst, const u8* __restrict__ src, int n
     } else {
         for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
     }
+}
+
+// Contiguous bytes shared -> global between any addresses that are equal
+// modulo 16: vectors between the unaligned ends.
+UP_DI void tile_bytes_out(u8* __restrict__ dst, const u8* __restrict__ src, int n) {
+    const int lead = (int)((16u - (u32)(unsigned long long)dst) & 15u), head = n < lead ? n : lead;
+    const int vecs = (n - head) >> 4, tail = head + (vecs << 4);
+    for (int i = threadIdx.x; i < head; i += blockDim.x) dst[i] = src[i];
+    const uint4* s = (const uint4*)(src + head);
+    uint4* d = (uint4*)(dst + head);
+    for (int i = threadIdx.x; i < vecs; i += blockDim.x) d[i] = s[i];
+    for (int i = tail + threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
 // ------------------------------------------- exact group accumulators
