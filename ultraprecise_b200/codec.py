@@ -8,6 +8,7 @@ metadata and are not stored.
 """
 from __future__ import annotations
 
+from functools import lru_cache
 from typing import Iterable, Sequence
 
 import numpy as np
@@ -15,6 +16,7 @@ import numpy as np
 from . import abi
 
 
+@lru_cache(maxsize=None)
 def compact_bytes(p: int) -> int:
     b = abi.load().up_compact_bytes(p)
     if b < 1:

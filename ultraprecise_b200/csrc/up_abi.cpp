@@ -1,6 +1,7 @@
 // up_abi.cpp — the C entry points of libultraprecise.so (include/ultraprecise.h).
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -101,27 +102,84 @@ int resident_ctas(void* kernel, int threads, int smem) {
     return n;
 }
 
-up_status set_smem(void* kernel, int smem) {
-    if (smem > 48 * 1024) {
-        UP_CUDA(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+// Shared memory above 48 KB is asked for once per kernel and device, together
+// with the CTAs per SM; 0: refused.
+template <int (*Find)(void*, int, int)>
+int prepared(void* kernel, int threads, int smem) {
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
-    return UP_OK;
+    return Find(kernel, threads, smem);
+}
+
+// CTAs of a looping launch: the resident ones of every SM of the current
+// device; <= 0 when there is no device or the kernel cannot run on it.
+template <int (*Find)(void*, int, int)>
+int64_t resident_grid(const up_module* m, void* kernel, int threads, int smem) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    const int sms = sm_count_current();
+    return sms <= 0 ? 0 : (int64_t)sms * jit_resident(*m->jm.ks, kernel, dev, threads, smem, prepared<Find>);
 }
 
 }  // namespace
 
 namespace upi {
 int sm_count_current() {
+    static std::atomic<int> known[64];  // SMs by device, 0 unknown
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
+    if (dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
+    if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
     return n;
+}
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64];  // by device, kept to the process's end
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    // an allocation under capture becomes a node that owns its memory: no pool
+    // is needed, and none is made while a stream captures
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) {
+        cudaGetLastError();
+        capturing = cudaStreamCaptureStatusActive;
+    }
+    cudaMemPool_t pool = nullptr;
+    if (dev < 64 && capturing == cudaStreamCaptureStatusNone) {
+        std::lock_guard<std::mutex> g(mu);
+        if (!pools[dev]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            uint64_t keep = kScratchKeep;
+            cudaMemPool_t made = nullptr;
+            if (cudaMemPoolCreate(&made, &props) == cudaSuccess &&
+                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
+                pools[dev] = made;
+            } else {
+                cudaGetLastError();
+                if (made) cudaMemPoolDestroy(made);
+            }
+        }
+        pool = pools[dev];
+    }
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
 }
 }  // namespace upi
 
@@ -206,15 +264,14 @@ up_status up_expr_launch_many(up_module* m, const up_column* in, int32_t n_in, c
         if (st != UP_OK) return st;
     }
     if (reqs.empty()) return UP_OK;
-    const int sms = sm_count_current();
-    if (sms <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
+    if (sm_count_current() <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
     void* k = jit_kernel(*m->jm.ks, "up_expr_multi");
     if (!k) return fail(UP_ERR_CUDA, "module has no up_expr_multi kernel");
-    up_status st = set_smem(k, g.multi_smem);
-    if (st != UP_OK) return st;
+    const int64_t cap = resident_grid<occupancy>(m, k, g.multi_threads, g.multi_smem);
+    if (cap <= 0) return fail(UP_ERR_CUDA, "shared memory of up_expr_multi refused");
     UpMultiReq* d = nullptr;
     const size_t bytes = reqs.size() * sizeof(UpMultiReq);
-    UP_CUDA(cudaMallocAsync((void**)&d, bytes, s));
+    UP_CUDA(scratch_alloc((void**)&d, bytes, s));
     cudaError_t e = cudaMemcpyAsync(d, reqs.data(), bytes, cudaMemcpyHostToDevice, s);
     UpMultiArgs a;
     memset(&a, 0, sizeof a);
@@ -223,7 +280,6 @@ up_status up_expr_launch_many(up_module* m, const up_column* in, int32_t n_in, c
     a.n_req = (int)reqs.size();
     void* args[1] = {&a};
     if (e == cudaSuccess) {
-        const int64_t cap = (int64_t)sms * occupancy(k, g.multi_threads, g.multi_smem);
         e = cudaLaunchKernel((const void*)k, dim3((unsigned)std::min<int64_t>(tiles, cap)), dim3(g.multi_threads),
                              args, (size_t)g.multi_smem, s);
     }
@@ -282,23 +338,22 @@ up_status expr_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64_
     a.out_nullable = g.out_bytes != (g.out_is_compare ? 1 : compact_bytes(g.out_precision));
     vec_ok = vec_ok && aligned16(out);
     a.vec_ok = vec_ok ? 1 : 0;
-    const int sms = sm_count_current();
-    if (sms <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
+    if (sm_count_current() <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
     void* args[1] = {&a};
     cudaStream_t s = (cudaStream_t)stream;
     if (contig && !a.out_nullable) {
         void* k = jit_kernel(*m->jm.ks, "up_expr_tile");
-        st = set_smem(k, g.smem_bytes);
-        if (st != UP_OK) return st;
         const int64_t ntiles = (rows + g.tile_rows - 1) / g.tile_rows;
-        const int64_t cap =
-            spread ? (int64_t)INT32_MAX : (int64_t)sms * resident_ctas(k, g.block_threads, g.smem_bytes);
+        const int64_t resident = resident_grid<resident_ctas>(m, k, g.block_threads, g.smem_bytes);
+        if (resident <= 0) return fail(UP_ERR_CUDA, "shared memory of up_expr_tile refused");
+        const int64_t cap = spread ? (int64_t)INT32_MAX : resident;
         const unsigned grid = (unsigned)std::min<int64_t>(ntiles, cap);
         UP_CUDA(cudaLaunchKernel((const void*)k, dim3(grid), dim3(g.block_threads), args, (size_t)g.smem_bytes, s));
     } else {
         void* k = jit_kernel(*m->jm.ks, "up_expr_generic");
         const int64_t blocks = (rows + g.block_threads - 1) / g.block_threads;
-        const int64_t cap = spread ? (int64_t)INT32_MAX : (int64_t)sms * occupancy(k, g.block_threads, 0) * 4;
+        const int64_t cap =
+            spread ? (int64_t)INT32_MAX : resident_grid<occupancy>(m, k, g.block_threads, 0) * 4;
         const unsigned grid = (unsigned)std::min<int64_t>(blocks, cap);
         UP_CUDA(cudaLaunchKernel((const void*)k, dim3(grid), dim3(g.block_threads), args, 0, s));
     }
@@ -450,8 +505,7 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
         if (!outs[k]) return fail(UP_ERR_INVALID_ARG, "output " + std::to_string(k) + " is NULL");
         a.out[k] = (uint8_t*)outs[k];
     }
-    const int sms = sm_count_current();
-    if (sms <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
+    if (sm_count_current() <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t accw = (size_t)std::max(g.acc_words_per_group, 1);
     size_t need = query_scratch_bytes(g, n_groups);
@@ -473,7 +527,7 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
                                                 std::to_string(need) + " bytes, " +
                                                 std::to_string(caller_scratch_bytes) + " given");
     } else {
-        UP_CUDA(cudaMallocAsync(&scratch, need, s));
+        UP_CUDA(scratch_alloc(&scratch, need, s));
     }
     cudaError_t e = cudaMemsetAsync(scratch, 0, need, s);
     a.rows = rows;
@@ -513,10 +567,10 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
                 const int threads = mode == 'r' ? g.q_threads_r : g.block_threads;
                 const int tile_rows = mode == 'r' ? g.q_tile_rows_r : g.q_tile_rows;
                 const int64_t ntiles = (rows + tile_rows - 1) / tile_rows;
-                if (set_smem(k, smem) != UP_OK) return cudaErrorInvalidValue;
                 // the register and shared-memory modes merge once per CTA, so a
                 // spread launch keeps a bounded grid of several waves
-                const int64_t cap = (int64_t)sms * occupancy(k, threads, smem) * (spread ? 8 : 1);
+                const int64_t cap = resident_grid<occupancy>(m, k, threads, smem) * (spread ? 8 : 1);
+                if (cap <= 0) return cudaErrorInvalidValue;
                 return cudaLaunchKernel((const void*)k, dim3((unsigned)std::min<int64_t>(ntiles, cap)),
                                         dim3(threads), args, (size_t)smem, s);
             };
@@ -533,7 +587,7 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
         } else {
             void* k = jit_kernel(*m->jm.ks, "up_query_acc");
             const int64_t blocks = (rows + g.block_threads - 1) / g.block_threads;
-            const int64_t cap = (int64_t)sms * occupancy(k, g.block_threads, 0) * 4;
+            const int64_t cap = resident_grid<occupancy>(m, k, g.block_threads, 0) * 4;
             e = cudaLaunchKernel((const void*)k, dim3((unsigned)std::min<int64_t>(blocks, cap)), dim3(g.block_threads),
                                  args, 0, s);
         }
@@ -591,7 +645,7 @@ up_status up_aggregate_column_data(const up_column* src, int32_t kind, const int
     cudaStream_t s = (cudaStream_t)stream;
     int32_t* gid = nullptr;
     if (rows > 0) {
-        UP_CUDA(cudaMallocAsync((void**)&gid, (size_t)rows * 4u, s));
+        UP_CUDA(scratch_alloc((void**)&gid, (size_t)rows * 4u, s));
         cudaError_t e = launch_fill_segment_gids(group_starts, n_groups, rows, gid, s);
         if (e != cudaSuccess) {
             cudaFreeAsync(gid, s);

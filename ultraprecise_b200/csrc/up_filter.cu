@@ -158,7 +158,7 @@ up_status up_filter_flags(const uint8_t* flags, int64_t rows, int32_t* indices, 
     }
     const int64_t nb = (rows + kTile - 1) / kTile;
     void* scratch = nullptr;
-    cudaError_t e = cudaMallocAsync(&scratch, (size_t)nb * (sizeof(int32_t) + sizeof(int64_t)) + 16, s);
+    cudaError_t e = scratch_alloc(&scratch, (size_t)nb * (sizeof(int32_t) + sizeof(int64_t)) + 16, s);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(e == cudaErrorMemoryAllocation ? UP_ERR_NO_MEMORY : UP_ERR_CUDA,

@@ -25,6 +25,7 @@
 #include <mutex>
 #include <sstream>
 #include <thread>
+#include <tuple>
 #include <unordered_map>
 
 #include <zlib.h>
@@ -49,6 +50,10 @@ struct JitKernelSet {
     std::vector<char> cubin;
     cudaLibrary_t lib = nullptr;
     std::map<std::string, cudaKernel_t> kernels;
+    // resident CTAs per SM of a kernel's launches, by device, threads and
+    // shared memory (found out at the first launch of each)
+    mutable std::mutex mu;
+    mutable std::map<std::tuple<void*, int, int, int>, int> resident;
     ~JitKernelSet() {
         if (lib) cudaLibraryUnload(lib);
     }
@@ -483,6 +488,17 @@ up_status jit_get(const GeneratedModule& gen, std::shared_ptr<JitKernelSet>& out
 void* jit_kernel(const JitKernelSet& ks, const std::string& name) {
     auto it = ks.kernels.find(name);
     return it == ks.kernels.end() ? nullptr : (void*)it->second;
+}
+
+int jit_resident(const JitKernelSet& ks, void* kernel, int device, int threads, int smem,
+                 int (*find)(void* kernel, int threads, int smem)) {
+    const auto key = std::make_tuple(kernel, device, threads, smem);
+    std::lock_guard<std::mutex> g(ks.mu);
+    auto it = ks.resident.find(key);
+    if (it != ks.resident.end()) return it->second;
+    const int n = find(kernel, threads, smem);
+    if (n > 0) ks.resident.emplace(key, n);
+    return n;
 }
 
 int jit_cache_size(bool clear) {

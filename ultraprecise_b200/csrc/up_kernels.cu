@@ -250,7 +250,7 @@ cudaError_t launch_group_table_small_keys_async(const void* const* key_cols, con
     int total = 0;
     const KeyCols k = key_cols_of(key_cols, key_bytes, n_keys, &total);
     void* scratch = nullptr;
-    cudaError_t e = cudaMallocAsync(&scratch, kKeyWords * 4, s);
+    cudaError_t e = scratch_alloc(&scratch, kKeyWords * 4, s);
     if (e != cudaSuccess) return e;
     e = group_table_async(k, total, rows, table, table + kTableCount, (u32*)scratch, group_keys, s);
     const cudaError_t e2 = cudaFreeAsync(scratch, s);
@@ -275,7 +275,7 @@ cudaError_t launch_group_ids_small_keys(const void* const* key_cols, const int32
     const KeyCols k = key_cols_of(key_cols, key_bytes, n_keys, &total);
     void* scratch = nullptr;
     // a whole key table (forward entries, id -> key list, count), then the bitmap
-    cudaError_t e = cudaMallocAsync(&scratch, (size_t)kTableEntries * 4 + kKeyWords * 4, s);
+    cudaError_t e = scratch_alloc(&scratch, (size_t)kTableEntries * 4 + kKeyWords * 4, s);
     if (e != cudaSuccess) return e;
     int32_t* table = (int32_t*)scratch;
     u32* bits = (u32*)((u8*)scratch + (size_t)kTableEntries * 4);

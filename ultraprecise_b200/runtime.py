@@ -63,17 +63,13 @@ class DeviceColumn:
         return self.data.numel() // self.value_bytes
 
     def up_column(self) -> abi.UpColumn:
-        c = abi.UpColumn()
-        c.data = self.data.data_ptr() if self.data is not None else None
-        c.blocks = self.block_ptrs.data_ptr() if self.blocks is not None else None
-        c.block_prefix = self.block_prefix.data_ptr() if self.blocks is not None else None
-        c.n_blocks = len(self.blocks) if self.blocks is not None else 0
-        c.indices = self.indices.data_ptr() if self.indices is not None else None
-        c.precision = self.precision
-        c.scale = self.scale
-        c.value_bytes = self.value_bytes
-        c.nullable = 1 if self.nullable else 0
-        return c
+        blocks = self.blocks is not None
+        return abi.UpColumn(self.data.data_ptr() if self.data is not None else None,
+                            self.block_ptrs.data_ptr() if blocks else None,
+                            self.block_prefix.data_ptr() if blocks else None,
+                            len(self.blocks) if blocks else 0,
+                            self.indices.data_ptr() if self.indices is not None else None,
+                            self.precision, self.scale, self.value_bytes, 1 if self.nullable else 0)
 
     @staticmethod
     def from_host(raw: bytes, precision: int, scale: int, device="cuda", nullable=False) -> "DeviceColumn":
@@ -86,10 +82,7 @@ class DeviceColumn:
 
 
 def _columns_array(cols: Sequence[DeviceColumn]):
-    arr = (abi.UpColumn * max(1, len(cols)))()
-    for i, c in enumerate(cols):
-        arr[i] = c.up_column()
-    return arr
+    return (abi.UpColumn * max(1, len(cols)))(*[c.up_column() for c in cols])
 
 
 class ExprModule:
