@@ -730,6 +730,7 @@ UP_DI void ld_compact_bytes(const u8* p, u32 (&m)[N], u32& sign) {
     m[TOPL] &= (TOPB == 31) ? 0x7fffffffu : ((1u << TOPB) - 1u);
 }
 
+#ifndef UP_HOST_TEST
 // Word loads of a B-byte value anywhere in device memory whose column starts
 // on a 4-byte boundary: the words around the value's start hold bytes of the
 // same column, the last bytes are read one by one unless the value fills
@@ -797,6 +798,7 @@ UP_DI void ld_compact(const u8* p, int words, u32 (&m)[N], u32& sign) {
     else if (words == 2) ld_compact_global<B, N>(p, m, sign);
     else ld_compact_bytes<B, N>(p, m, sign);
 }
+#endif  // UP_HOST_TEST
 
 // Overflow test: any magnitude bit at or above 8*B-1 would be lost or would
 // collide with the sign bit.
@@ -1632,6 +1634,7 @@ UP_DI void atomic_acc_add(u32* acc, const u32 (&m)[N], u32 sign) {
     atomic_add_twos(acc, t);
 }
 
+#ifndef UP_HOST_TEST
 // Cell accumulators: a group's running sum held as signed 16-bit pieces of
 // the magnitude, one 32-bit cell per piece in shared memory, S cells apart.
 // Adding a value is one atomic without a returned value and without a carry
@@ -1711,7 +1714,6 @@ struct RSum<3> {
     UP_DI void reduce_into(int* pieces, int lane);
 };
 
-#ifndef UP_HOST_TEST
 // A warp's register sums into 16-bit pieces in shared memory (the top piece
 // signed): a CTA's 32 warps keep every piece below 2^26.
 template <int W>
@@ -1753,7 +1755,6 @@ UP_DI void ld_quad(u32 (&w)[B], const u8* p) {
         for (int i = 0; i < B; i++) w[i] = *(const u32*)(p + 4 * i);
     }
 }
-#endif
 
 // 32 bits at byte offset o (a compile-time constant after unrolling)
 template <int W>
@@ -1793,6 +1794,7 @@ UP_DI void limb_sums_add(i64* acc, const u32 (&m)[N], u32 sign) {
     for (int i = 0; i < N; i++)
         if (m[i]) atomicAdd((u64*)(acc + i), (u64)(sign ? -(i64)m[i] : (i64)m[i]));
 }
+#endif  // UP_HOST_TEST
 
 // The reference's nullable_type<Decimal> image of a SUM/AVG result
 // (decimal.hxx:130-140 plus the leading flag; kernel_segreduce.hxx:609-612):
