@@ -271,10 +271,44 @@ struct TEmitter {
     const std::vector<NodeFacts>& f;
     int T, K;
     std::ostringstream body, globals;
-    std::set<int> p10;
+    std::set<int> p10, tc_p10;
     int tmp = 0;
     bool out_of_line = false;  // call multiplies and divisions out of line
     bool words = false;        // columns come from a padded shared-memory tile (word loads)
+    bool tensor = false;       // wide products on the tensor cores, through a warp's scratch `ws`
+    int scratch_words = 0;     // of a warp, for the products emitted so far
+
+    // Operand limbs from which a product goes to the tensor cores: the window
+    // product costs a step of shuffles per limb of the shorter operand, the
+    // tensor one a nearly fixed number of instructions.
+    static constexpr int kTensorMinLimbs = 6;
+    bool on_tensor(int lb) const { return tensor && !out_of_line && K % 4 == 0 && K <= 16 && lb >= kTensorMinLimbs; }
+    static int tc_steps(int lb) { return (4 * lb + 7 + 31) / 32; }
+    static int tc_copy(int lb) {
+        const int n = (8 * tc_steps(lb) + 4 + 7) / 8;
+        return 8 * (n % 2 ? n : n + 1);
+    }
+    // words of a warp's scratch for a product (tc_words of the device header)
+    int tc_words(int la, int lb, bool constant) const {
+        const int aw = (16 + std::max(la + 20, T * K) + 3) / 4 * 4;
+        const int out = ((la + lb + 1) / 2 + 15) / 16 * 64;
+        return 32 / T * (aw + std::max(out, constant ? 0 : 4 * tc_copy(lb)));
+    }
+    // the shifted copies of a constant as tc_stage_b lays them out
+    std::string tc_constant(const std::string& name, const Big& p) {
+        const int lb = (int)p.m.size(), cs = tc_copy(lb);
+        auto limb = [&](int i) { return i >= 0 && i < lb ? p.m[i] : 0u; };
+        std::ostringstream o;
+        o << "__device__ const u32 " << name << "[" << 4 * cs << "] = {";
+        for (int s = 0; s < 4; s++)
+            for (int i = 0; i < cs; i++) {
+                const int w = i - 4;
+                const uint32_t x = s ? (limb(w) >> (8 * s)) | (limb(w + 1) << (32 - 8 * s)) : limb(w);
+                o << (s || i ? ", " : "") << hex32(x);
+            }
+        o << "};\n";
+        return o.str();
+    }
 
     TEmitter(const up_expr_node* n, const up_col_type* c, const std::vector<NodeFacts>& facts, int t, int k)
         : nodes(n), cols(c), f(facts), T(t), K(k) {}
@@ -305,6 +339,15 @@ struct TEmitter {
         const int d = sc - f[a].scale;
         const Big p = big_pow10(d);
         std::string t = "t" + std::to_string(tmp++);
+        const int np = (int)p.m.size();
+        if (on_tensor(np) && f[a].limbs >= np) {
+            const std::string c = "TC10_" + std::to_string(d);
+            if (tc_p10.insert(d).second) globals << tc_constant(c, p);
+            scratch_words = std::max(scratch_words, tc_words(f[a].limbs, np, true));
+            body << "    u32 " << t << "[" << K << "]; tpi_mul_const<" << tk() << ", " << f[a].limbs << ", " << np << ">(" << t
+                 << ", " << v(a) << ", " << c << ", ws);\n";
+            return t;
+        }
         body << "    u32 " << t << "[" << K << "]; tpi_mul_const<" << tk() << ", " << f[a].limbs << ", " << p.m.size()
              << ">(" << t << ", " << v(a) << ", " << p10_name(d) << ");\n";
         return t;
@@ -354,6 +397,13 @@ struct TEmitter {
                 // the operand with fewer limbs is streamed limb by limb
                 int a = nd.left, b = nd.right;
                 if (f[a].limbs < f[b].limbs) std::swap(a, b);
+                if (on_tensor(f[b].limbs)) {
+                    scratch_words = std::max(scratch_words, tc_words(f[a].limbs, f[b].limbs, false));
+                    body << "    u32 " << v(k) << "[" << K << "]; tpi_mul<" << tk() << ", " << f[a].limbs << ", " << f[b].limbs
+                         << ">(" << v(k) << ", " << v(a) << ", " << v(b) << ", ws); u32 " << s(k) << " = " << s(nd.left)
+                         << " ^ " << s(nd.right) << ";\n";
+                    break;
+                }
                 body << "    u32 " << v(k) << "[" << K << "]; tpi_mul" << ni() << "<" << tk() << ", " << f[a].limbs << ", "
                      << f[b].limbs
                      << ">(" << v(k)
@@ -673,6 +723,12 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
             if (t > 1) tpiT = t;
         }
         if (tpiT > 0) tpiK = (w + tpiT - 1) / tpiT;
+        // whole groups of four limbs per thread where a product takes the tensor cores
+        if (tpiK >= 3 && tpiK <= 16)
+            for (int k : topo)
+                if (nodes[k].kind == UP_NODE_MUL &&
+                    std::min(f[nodes[k].left].limbs, f[nodes[k].right].limbs) >= TEmitter::kTensorMinLimbs)
+                    tpiK = (tpiK + 3) / 4 * 4;
     }
     out.threads_per_value = tpiT > 0 ? tpiT : 1;
 
@@ -681,6 +737,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
     if (tpiT > 0) {
         TEmitter te(nodes, cols, f, tpiT, tpiK);
         te.words = true;  // the columns are read from the staged tile below (padded by 16 bytes)
+        te.tensor = true;
         te.plan(topo);
         for (int k : topo) te.node(k);
         const int CT = 256;               // CTA threads
@@ -694,8 +751,11 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         }
         const int off_out = smem;
         smem += ((R * BO + 16 + 15) / 16) * 16;
+        const int off_ws = smem;  // the warps' scratch for products on the tensor cores
+        const int ws_words = (te.scratch_words + 3) / 4 * 4;
+        smem += CT / 32 * ws_words * 4;
         src << te.globals.str();
-        src << "UP_DI u32 up_trow(" << params_decl(used) << "u8* __restrict__ out, const bool store) {\n";
+        src << "UP_DI u32 up_trow(" << params_decl(used) << "u8* __restrict__ out, const bool store, u32* ws) {\n";
         src << "    u32 err = 0u;\n" << te.constants() << te.body.str();
         if (cmp_root)
             src << "    if (store && tpi_rank<" << tpiT << ">() == 0) out[0] = (u8)c" << root << ";\n";
@@ -704,8 +764,10 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
                 << ", store);\n";
         src << "    return err;\n}\n\n";
         // four CTAs per SM (at most 64 registers): measured on B200, p=600
-        // a*b+c at 16 threads per value 2.27 -> 2.17 ms
-        src << "extern \"C\" __global__ void __launch_bounds__(" << CT << ", 4) up_expr_tile(const UpArgs a) {\n";
+        // a*b+c at 16 threads per value with window products 2.27 -> 2.17 ms;
+        // two (128 registers) for the fragments of tensor products
+        src << "extern \"C\" __global__ void __launch_bounds__(" << CT << ", " << (ws_words ? 2 : 4)
+            << ") up_expr_tile(const UpArgs a) {\n";
         src << "    extern __shared__ __align__(16) u8 sm[];\n";
         src << "    constexpr int R = " << R << ";\n    constexpr int G = " << G << ";\n";
         src << "    const int grp = (int)threadIdx.x / " << tpiT << ";\n";
@@ -727,7 +789,8 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         src << "            const u32 e = up_trow(";
         for (size_t i = 0; i < used.size(); i++)
             src << "sm + " << off[i] << " + rr * " << compact_bytes(cols[used[i]].precision) << ", ";
-        src << "sm + " << off_out << " + rr * " << BO << ", valid);\n";
+        src << "sm + " << off_out << " + rr * " << BO << ", valid, (u32*)(sm + " << off_ws << ") + (threadIdx.x >> 5) * "
+            << ws_words << ");\n";
         src << "            if (valid) err |= e;\n        }\n";
         src << "        __syncthreads();\n";
         src << "        tile_copy_out(a.out + row0 * " << BO << ", sm + " << off_out << ", nr * " << BO

@@ -1113,6 +1113,191 @@ UP_DI void tpi_mul_const(u32 (&r)[K], const u32 (&a)[K], const u32 (&p)[NP]) {
     tpi_window_out<T, K, KA, NP>(r, acc, e);
 }
 
+// ---------------------------------------- products on the tensor cores
+// A product of two spread values is a convolution of their bytes,
+// c[m] = sum_j a[m-j] b[j], and with m = 8u + v and j = v + l a matrix product
+//   C[u][v] = sum_l A[u][l] B[l][v],  A[u][l] = a[8u - l],  B[l][v] = b[v + l],
+// l = -7 .. 4*LB-1, on mma.m16n8k32 with u8 operands and s32 sums (exact: a sum
+// is below 255^2 * 4 * LB < 2^31).  The step of 8 bytes per row makes every A
+// fragment word one byte-swapped limb of a at index 2u - (l + 7 - 8) / 4, so a
+// lane's fragments of all tiles and steps are one sequence X(j) of words; B
+// fragments come from four copies of b shifted by 0..3 bytes.  The eight
+// positions of a row u are spread over a quad: after exchanging halves every
+// lane holds one limb's sum (below 2^51) per tile.  The limb sums go through
+// the warp's scratch back to the spread layout, where carries resolve as in
+// tpi_add.  The warp's 32 / T values run one after the other.
+// Against the window product: 32 limb steps of shuffles and a wide multiply
+// each become a few tensor instructions.
+__host__ __device__ constexpr int tc_steps(int lb) { return (4 * lb + 7 + 31) / 32; }
+// words between the shifted copies: an odd multiple of 8, so that the four
+// copies' reads fall into different banks
+__host__ __device__ constexpr int tc_copy(int lb) { return (8 * tc_steps(lb) + 4 + 7) / 8 % 2 ? (8 * tc_steps(lb) + 4 + 7) / 8 * 8 : (8 * tc_steps(lb) + 4 + 7) / 8 * 8 + 8; }
+__host__ __device__ constexpr int tc_tiles(int la, int lb) { return ((la + lb + 1) / 2 + 15) / 16; }
+__host__ __device__ constexpr int tc_a_words(int t, int k, int la) { return (16 + (la + 20 > t * k ? la + 20 : t * k) + 3) / 4 * 4; }
+__host__ __device__ constexpr int tc_b_words(int la, int lb, bool constant) {
+    const int out = tc_tiles(la, lb) * 64, copies = constant ? 0 : 4 * tc_copy(lb);
+    return copies > out ? copies : out;
+}
+// scratch words of a warp for one product
+__host__ __device__ constexpr int tc_words(int t, int k, int la, int lb, bool constant) {
+    return 32 / t * (tc_a_words(t, k, la) + tc_b_words(la, lb, constant));
+}
+
+UP_DI void mma_u8(int (&c)[4], u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// The byte-swapped limbs of every value of the warp, zeros around them.
+template <int T, int K, int LA, int VW>
+UP_DI void tc_stage_a(u32* ws, const u32 (&a)[K]) {
+    static_assert(K % 4 == 0, "limbs move in groups of four");
+    constexpr int AW = tc_a_words(T, K, LA);
+    const int g = tpi_rank<T>();
+    u32* A = ws + (int)((threadIdx.x & 31u) / T) * VW;
+#pragma unroll
+    for (int i = 0; i < K; i += 4)
+        *(uint4*)(A + 16 + g * K + i) = make_uint4(__byte_perm(a[i], 0u, 0x0123u), __byte_perm(a[i + 1], 0u, 0x0123u),
+                                                   __byte_perm(a[i + 2], 0u, 0x0123u), __byte_perm(a[i + 3], 0u, 0x0123u));
+    for (int i = g; i < 16; i += T) A[i] = 0u;
+    for (int i = 16 + T * K + g; i < AW; i += T) A[i] = 0u;
+}
+
+// The four shifted copies of every value of the warp: copy s, word 4 + w =
+// bytes 4w + s .. 4w + s + 3.
+template <int T, int K, int LB, int VW, int AW>
+UP_DI void tc_stage_b(u32* ws, const u32 (&b)[K]) {
+    constexpr int CS = tc_copy(LB);
+    const int g = tpi_rank<T>();
+    u32* B = ws + (int)((threadIdx.x & 31u) / T) * VW + AW;
+    u32 above = __shfl_down_sync(kFull, b[0], 1, T);
+    if (g == T - 1) above = 0u;
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+#pragma unroll
+        for (int i = 0; i < K; i += 4) {
+            u32 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                x[j] = __funnelshift_r(b[i + j], i + j + 1 < K ? b[i + j + 1 < K ? i + j + 1 : 0] : above, 8u * s);
+            if (g * K + i < LB) *(uint4*)(B + s * CS + 4 + g * K + i) = make_uint4(x[0], x[1], x[2], x[3]);
+        }
+        if (g == 0) {
+            B[s * CS + 2] = 0u;
+            B[s * CS + 3] = s ? b[0] << (32 - 8 * s) : 0u;
+        }
+        for (int i = 4 + (LB + 3) / 4 * 4 + g; i < CS; i += T) B[s * CS + i] = 0u;
+    }
+}
+
+// The product's limb sums of every value of the warp from staged operands;
+// with CONST the B words are those of a constant (bc, laid out like a copy
+// set, in device memory), the same for all values.
+template <int T, int K, int LA, int LB, bool CONST>
+UP_DI void tc_limb_sums(u32* ws, const u32* __restrict__ bc) {
+    constexpr int AW = tc_a_words(T, K, LA), VW = AW + tc_b_words(LA, LB, CONST);
+    constexpr int KS = tc_steps(LB), MT = tc_tiles(LA, LB), CS = tc_copy(LB);
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int sh = (g - 7) & 3, q = (g - 7) >> 2;  // b's byte g - 7 is byte sh of word q
+    const int b_off = sh * CS + 4 + q + t, a_off = 16 + 2 * g + 1 - t;
+    u32 bw[2 * KS];
+    if constexpr (CONST) {
+#pragma unroll
+        for (int k = 0; k < 2 * KS; k++) bw[k] = __ldg(bc + b_off + 4 * k);
+    }
+#pragma unroll 1
+    for (int v = 0; v < 32 / T; v++) {
+        const u32* A = ws + v * VW + a_off;
+        u32* B = ws + v * VW + AW;
+        if constexpr (!CONST) {
+#pragma unroll
+            for (int k = 0; k < 2 * KS; k++) bw[k] = B[b_off + 4 * k];
+        }
+        // X(j) = limb 2g + 1 - t + 4j: nonzero only for -3 <= j <= (LA + 1) / 4
+        constexpr int JLO = -3, JN = (LA + 1) / 4 + 4;
+        u32 xs[JN];
+#pragma unroll
+        for (int j = 0; j < JN; j++) xs[j] = A[4 * (j + JLO)];
+        int c[MT][4];
+#pragma unroll
+        for (int m = 0; m < MT; m++) c[m][0] = c[m][1] = c[m][2] = c[m][3] = 0;
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int k = 0; k < KS; k++) {
+                const int j = 8 * m - 2 * k - JLO;  // index of a0's words
+                if (j + 4 >= 0 && j - 1 < JN) {
+                    auto x = [&](int i) { return i >= 0 && i < JN ? xs[i >= 0 && i < JN ? i : 0] : 0u; };
+                    mma_u8(c[m], x(j), x(j + 4), x(j - 1), x(j + 3), bw[2 * k], bw[2 * k + 1]);
+                }
+            }
+        __syncwarp();  // every lane has read this value's operands: the sums may take b's place
+        u64* o = (u64*)B;
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+            const u64 w0 = (u64)(u32)c[m][1] * 256u + (u32)c[m][0], w1 = (u64)(u32)c[m][3] * 256u + (u32)c[m][2];
+            const bool odd = t & 1;
+            const u64 send = odd ? w0 : w1, keep = odd ? w1 : w0;
+            const u64 recv = __shfl_xor_sync(kFull, send, 1);
+            const u64 lo = odd ? recv : keep, hi = odd ? keep : recv;
+            o[2 * (16 * m + (odd ? 8 : 0) + g) + (t >> 1)] = lo + (hi << 16);
+        }
+    }
+    __syncwarp();
+}
+
+// The limb sums back in the spread layout, carries resolved (low T*K limbs).
+template <int T, int K, int LA, int LB, bool CONST>
+UP_DI void tc_collect(u32 (&r)[K], const u32* ws) {
+    constexpr int AW = tc_a_words(T, K, LA), VW = AW + tc_b_words(LA, LB, CONST), NL = tc_tiles(LA, LB) * 32;
+    const int g = tpi_rank<T>();
+    const u64* o = (const u64*)(ws + (int)((threadIdx.x & 31u) / T) * VW + AW);
+    u64 c = 0;
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        if (g * K + i < NL) c += o[g * K + i];
+        r[i] = (u32)c;
+        c >>= 32;
+    }
+    u32 in = __shfl_up_sync(kFull, (u32)c, 1, T);  // below 2^20
+    if (g == 0) in = 0u;
+    c = in;
+    u32 all = kFull;
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        c += r[i];
+        r[i] = (u32)c;
+        c >>= 32;
+        all &= r[i];
+    }
+    tpi_inc_local(r, tpi_carry_in<T>(c != 0, all == kFull));
+    __syncwarp();  // the scratch is free again
+}
+
+// r = a * b as tpi_mul (a at most LA, b at most LB nonzero limbs), through
+// the warp's scratch of tc_words words (16-byte aligned).
+template <int T, int K, int LA, int LB>
+UP_DI void tpi_mul(u32 (&r)[K], const u32 (&a)[K], const u32 (&b)[K], u32* ws) {
+    constexpr int AW = tc_a_words(T, K, LA), VW = AW + tc_b_words(LA, LB, false);
+    tc_stage_a<T, K, LA, VW>(ws, a);
+    tc_stage_b<T, K, LB, VW, AW>(ws, b);
+    __syncwarp();
+    tc_limb_sums<T, K, LA, LB, false>(ws, nullptr);
+    tc_collect<T, K, LA, LB, false>(r, ws);
+}
+
+// r = a * p for a constant of NP limbs whose shifted copies (laid out as
+// tc_stage_b leaves them) are at pc in device memory.
+template <int T, int K, int LA, int NP>
+UP_DI void tpi_mul_const(u32 (&r)[K], const u32 (&a)[K], const u32* __restrict__ pc, u32* ws) {
+    constexpr int VW = tc_a_words(T, K, LA) + tc_b_words(LA, NP, true);
+    tc_stage_a<T, K, LA, VW>(ws, a);
+    __syncwarp();
+    tc_limb_sums<T, K, LA, NP, true>(ws, pc);
+    tc_collect<T, K, LA, NP, true>(r, ws);
+}
+
 // Limb `pos` (the same position on every thread of the group; 0 when out of
 // range) broadcast to the whole group.
 template <int T, int K>
