@@ -699,7 +699,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
     if (cmp_root) {
         src << "    out[0] = (u8)c" << root << ";\n";
     } else if (BO % 4 == 0) {
-        src << "    if (words == 1) err |= st_compact_words<" << BO << ">(out, v" << root << ", s" << root << ");\n";
+        src << "    if (words == 3) err |= st_compact_words<" << BO << ">(out, v" << root << ", s" << root << ");\n";
         src << "    else err |= st_compact_bytes<" << BO << ">(out, v" << root << ", s" << root << ");\n";
     } else {
         src << "    err |= st_compact_bytes<" << BO << ">(out, v" << root << ", s" << root << ");\n";
@@ -861,7 +861,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
             int B = compact_bytes(cols[used[i]].precision);
             src << "in + " << off[i] << " + r * " << B << ", ";
         }
-        src << "ob + r * " << BO << ", true);\n";
+        src << "ob + r * " << BO << ", 3);\n";
         src << "        if (bulk) {\n";
         src << "            fence_async_smem();\n";
         src << "            __syncthreads();\n";
@@ -925,7 +925,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
             int B = compact_bytes(cols[used[i]].precision);
             src << "sm + " << off[i] << " + r * " << B << ", ";
         }
-        src << "sm + " << off_out << " + r * " << BO << ", true);\n";
+        src << "sm + " << off_out << " + r * " << BO << ", 3);\n";
         src << "        __syncthreads();\n";
         src << "        tile_copy_out(a.out + row0 * " << BO << ", sm + " << off_out << ", nr * " << BO
             << ", a.vec_ok != 0);\n";
@@ -969,7 +969,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         src << "        for (int r = threadIdx.x; r < nr; r += blockDim.x)\n            err |= up_row(";
         for (size_t i = 0; i < used.size(); i++)
             src << "sm + " << moff[i] << " + r * " << compact_bytes(cols[used[i]].precision) << ", ";
-        src << "sm + " << moff_out << " + r * " << BO << ", true);\n";
+        src << "sm + " << moff_out << " + r * " << BO << ", 3);\n";
         src << "        __syncthreads();\n";
         src << "        tile_copy_out(q.out + row0 * " << BO << ", sm + " << moff_out << ", nr * " << BO
             << ", q.vec_ok != 0);\n";
@@ -1604,7 +1604,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
             src << "            err |= up_qmags(";
             for (size_t i = 0; i < used.size(); i++)
                 src << "in + " << off[i] << " + r * " << compact_bytes(cols[used[i]].precision) << ", ";
-            src << "true" << margs() << ");\n";
+            src << "3" << margs() << ");\n";
         }
         src << "            const int s = hashed ? cell_slot<S>(tags, g) : g * rep + (lane & (rep - 1));\n";
         src << "            if (s >= 0) {\n                int* c = cells + s;\n";
@@ -1639,7 +1639,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
             src << "            err |= up_qvals(";
             for (size_t i = 0; i < used.size(); i++)
                 src << "in + " << off[i] << " + r * " << compact_bytes(cols[used[i]].precision) << ", ";
-            src << "true" << targs() << ");\n";
+            src << "3" << targs() << ");\n";
         }
         src << "            atomicAdd(a.cnt + g, 1ull);\n";
         for (int i = 0; i < NR; i++)
@@ -1746,7 +1746,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
                 src << "                err |= up_qmags(";
                 for (size_t i = 0; i < used.size(); i++)
                     src << "in + " << sr.off[i] << " + r * " << compact_bytes(cols[used[i]].precision) << ", ";
-                src << "true" << margs() << ");\n";
+                src << "3" << margs() << ");\n";
             }
             src << "                int* c = cells + j * 32 + lane;\n";
             for (int i = 0; i < NR; i++)

@@ -84,41 +84,110 @@ UP_DI int cmp(const u32 (&a)[NA], const u32 (&b)[NB]) {
     return r;
 }
 
+// Carry chains: one add, or one 32x32+64 multiply-add (the lo/hi pair of
+// neighbouring limbs), per instruction, the carry in the condition code from
+// one statement to the next.  64-bit sums of one limb at a time, which is what
+// plain C++ says, cost several instructions per limb.  The statements are
+// volatile, so they stay in order; nothing between the first and the last of
+// a chain touches the condition code.  Values of at most kPlainLimbs limbs (and
+// products of at most kPlainPairs) keep the plain form, which the compiler may
+// interleave with its neighbours: a*b+c at p=18 is bound by the latency of a
+// tile there (0.111 ms plain, 0.121 ms with chains on B200).
+constexpr int kPlainLimbs = 4, kPlainPairs = 6;
+#if defined(__CUDA_ARCH__)
+#define UP_CC3(NAME, INS)                                                                        \
+    UP_DI u32 NAME(u32 a, u32 b, u32 c) {                                                        \
+        u32 r;                                                                                   \
+        asm volatile(INS ".u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));             \
+        return r;                                                                                \
+    }
+#define UP_CC2(NAME, INS)                                                             \
+    UP_DI u32 NAME(u32 a, u32 b) {                                                    \
+        u32 r;                                                                        \
+        asm volatile(INS ".u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));              \
+        return r;                                                                     \
+    }
+UP_CC3(mad_lo_cc, "mad.lo.cc")
+UP_CC3(madc_lo_cc, "madc.lo.cc")
+UP_CC3(madc_hi_cc, "madc.hi.cc")
+UP_CC2(add_cc, "add.cc")
+UP_CC2(addc_cc, "addc.cc")
+UP_CC2(addc, "addc")
+UP_CC2(sub_cc, "sub.cc")
+UP_CC2(subc_cc, "subc.cc")
+UP_CC2(subc, "subc")
+#undef UP_CC3
+#undef UP_CC2
+#else  // the host build: the same with a carry of its own
+static u32 cc_host = 0;
+UP_DI u32 cc_set(u64 s) {
+    cc_host = (u32)(s >> 32) & 1u;
+    return (u32)s;
+}
+UP_DI u32 mad_lo_cc(u32 a, u32 b, u32 c) { return cc_set((u64)(u32)((u64)a * b) + c); }
+UP_DI u32 madc_lo_cc(u32 a, u32 b, u32 c) { return cc_set((u64)(u32)((u64)a * b) + c + cc_host); }
+UP_DI u32 madc_hi_cc(u32 a, u32 b, u32 c) { return cc_set((((u64)a * b) >> 32) + c + cc_host); }
+UP_DI u32 add_cc(u32 a, u32 b) { return cc_set((u64)a + b); }
+UP_DI u32 addc_cc(u32 a, u32 b) { return cc_set((u64)a + b + cc_host); }
+UP_DI u32 addc(u32 a, u32 b) { return a + b + cc_host; }
+UP_DI u32 sub_cc(u32 a, u32 b) { return cc_set((u64)a - b); }
+UP_DI u32 subc_cc(u32 a, u32 b) { return cc_set((u64)a - b - cc_host); }
+UP_DI u32 subc(u32 a, u32 b) { return a - b - cc_host; }
+#endif
+
 // r = a + b over N limbs; returns the carry out of limb N-1
 template <int N, int NA, int NB>
 UP_DI u32 add(u32 (&r)[N], const u32 (&a)[NA], const u32 (&b)[NB]) {
-    u64 c = 0;
+    if constexpr (N <= kPlainLimbs) {
+        u64 c = 0;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        c += (u64)at(a, i) + at(b, i);
-        r[i] = (u32)c;
-        c >>= 32;
+        for (int i = 0; i < N; i++) {
+            c += (u64)at(a, i) + at(b, i);
+            r[i] = (u32)c;
+            c >>= 32;
+        }
+        return (u32)c;
     }
-    return (u32)c;
+    r[0] = add_cc(a[0], b[0]);
+#pragma unroll
+    for (int i = 1; i < N; i++) r[i] = addc_cc(at(a, i), at(b, i));
+    return addc(0u, 0u);
 }
 
 // r = a - b over N limbs (two's complement); returns 1 when a < b
 template <int N, int NA, int NB>
 UP_DI u32 sub(u32 (&r)[N], const u32 (&a)[NA], const u32 (&b)[NB]) {
-    u64 c = 1;
+    r[0] = sub_cc(a[0], b[0]);
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        c += (u64)at(a, i) + (u64)(~at(b, i));
-        r[i] = (u32)c;
-        c >>= 32;
-    }
-    return (u32)(c ^ 1u);
+    for (int i = 1; i < N; i++) r[i] = subc_cc(at(a, i), at(b, i));
+    return subc(0u, 0u) & 1u;
+}
+
+// a < b (magnitudes)
+template <int NA, int NB>
+UP_DI bool less(const u32 (&a)[NA], const u32 (&b)[NB]) {
+    constexpr int M = NA > NB ? NA : NB;
+    sub_cc(a[0], b[0]);
+#pragma unroll
+    for (int i = 1; i < M; i++) subc_cc(at(a, i), at(b, i));
+    return subc(0u, 0u) != 0u;
 }
 
 template <int N>
 UP_DI void negate(u32 (&r)[N]) {
-    u64 c = 1;
+    if constexpr (N <= kPlainLimbs) {
+        u64 c = 1;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        c += (u64)(~r[i]);
-        r[i] = (u32)c;
-        c >>= 32;
+        for (int i = 0; i < N; i++) {
+            c += (u64)(~r[i]);
+            r[i] = (u32)c;
+            c >>= 32;
+        }
+        return;
     }
+    r[0] = sub_cc(0u, r[0]);
+#pragma unroll
+    for (int i = 1; i < N; i++) r[i] = subc_cc(0u, r[i]);
 }
 
 // r += k (small), over N limbs
@@ -140,52 +209,107 @@ UP_DI void add_small(u32 (&r)[N], u32 k) {
 // operator-= rules, AriesDecimal.hxx:234-289, reduce to exactly that).
 template <int N, int NA, int NB>
 UP_DI void add_signed(u32 (&r)[N], u32& sr, const u32 (&a)[NA], u32 sa, const u32 (&b)[NB], u32 sb) {
+    // a + b, or a + ~b + 1; no carry out of the latter: a < b
     const bool same = sa == sb;
     const u32 x = same ? 0u : 0xffffffffu;
-    u64 c = same ? 0u : 1u;
+    u32 c;
+    if constexpr (N <= kPlainLimbs) {
+        u64 s = same ? 0u : 1u;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        c += (u64)at(a, i) + (u64)(at(b, i) ^ x);
-        r[i] = (u32)c;
-        c >>= 32;
+        for (int i = 0; i < N; i++) {
+            s += (u64)at(a, i) + (u64)(at(b, i) ^ x);
+            r[i] = (u32)s;
+            s >>= 32;
+        }
+        c = (u32)s;
+    } else {
+        add_cc(x, x);  // the carry in
+#pragma unroll
+        for (int i = 0; i < N; i++) r[i] = addc_cc(at(a, i), at(b, i) ^ x);
+        c = addc(0u, 0u);
     }
-    const bool neg = !same && c == 0u;  // a < b
+    const bool neg = !same && c == 0u;
     if (neg) negate(r);
     const bool nz = !is_zero(r);
     sr = same ? sa : (nz ? (neg ? sb : (sb ^ 1u)) : 0u);
 }
 
+// Half a row of a product: x += a[j] * k at limbs i + j for every second j
+// from J0 (low N limbs).  Neighbouring products fill neighbouring pairs of
+// limbs, so the half row is one chain, its carry ends in the limb above.
+template <int J0, int N, int NA>
+UP_DI void mul_row(u32 (&x)[N], const u32 (&a)[NA], u32 k, int i) {
+    int top = -1;
+#pragma unroll
+    for (int j = J0; j < NA; j += 2) {
+        const int l = i + j;
+        if (l < N) {
+            x[l < N ? l : 0] = j == J0 ? mad_lo_cc(a[j], k, x[l < N ? l : 0]) : madc_lo_cc(a[j], k, x[l < N ? l : 0]);
+            if (l + 1 < N) x[l + 1 < N ? l + 1 : 0] = madc_hi_cc(a[j], k, x[l + 1 < N ? l + 1 : 0]);
+        }
+        top = l + 2;
+    }
+    if (top >= 0 && top < N) x[top >= 0 && top < N ? top : 0] = addc(x[top >= 0 && top < N ? top : 0], 0u);
+}
+
+// r = a * b (low N limbs of the product), a row per limb of b: the even and
+// then the odd products of the row, each a carry chain of one wide
+// multiply-add per product.  Measured on B200 against 64-bit sums per limb:
+// the series at p=100 0.86 -> 0.70 ms, a/b at p=38 0.306 -> 0.282 ms.
+template <int N, int NA, int NB>
+UP_DI void mul_rows(u32 (&r)[N], const u32 (&a)[NA], const u32 (&b)[NB]) {
+    zero(r);
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+        if (i < N) {
+            mul_row<0>(r, a, b[i], i);
+            mul_row<1>(r, a, b[i], i);
+        }
+    }
+}
+
 // r = a * b (low N limbs of the product)
 template <int N, int NA, int NB>
 UP_DI void mul(u32 (&r)[N], const u32 (&a)[NA], const u32 (&b)[NB]) {
-    zero(r);
-    // products above UP_MUL_UNROLL_PAIRS limb pairs keep the outer loop rolled
-    // (compile time)
-#pragma unroll((NA * NB <= kMulUnrollPairs) ? NA : 1)
-    for (int i = 0; i < NA; i++) {
-        if (i >= N) break;
-        u64 c = 0;
+    if constexpr (NA * NB > kPlainPairs && NA * NB <= kMulUnrollPairs) {
+        if constexpr (NA >= NB) mul_rows(r, a, b);
+        else mul_rows(r, b, a);
+    } else {
+        // products above UP_MUL_UNROLL_PAIRS limb pairs keep the outer loop
+        // rolled (compile time)
+        zero(r);
+#pragma unroll((NA * NB <= kPlainPairs) ? NA : 1)
+        for (int i = 0; i < NA; i++) {
+            if (i >= N) break;
+            u64 c = 0;
 #pragma unroll
-        for (int j = 0; j < NB; j++) {
-            if (i + j < N) {
-                u64 t = (u64)a[i] * b[j] + r[i + j] + c;
-                r[i + j] = (u32)t;
-                c = t >> 32;
+            for (int j = 0; j < NB; j++) {
+                if (i + j < N) {
+                    u64 t = (u64)a[i] * b[j] + r[i + j] + c;
+                    r[i + j] = (u32)t;
+                    c = t >> 32;
+                }
             }
+            if (i + NB < N) r[i + NB] = (u32)c;
         }
-        if (i + NB < N) r[i + NB] = (u32)c;
     }
 }
 
 // r = a * k (k one limb)
 template <int N, int NA>
 UP_DI void mul_u32(u32 (&r)[N], const u32 (&a)[NA], u32 k) {
-    u64 c = 0;
+    if constexpr (NA <= kPlainLimbs) {
+        u64 c = 0;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        u64 t = (u64)at(a, i) * k + c;
-        r[i] = (u32)t;
-        c = t >> 32;
+        for (int i = 0; i < N; i++) {
+            u64 t = (u64)at(a, i) * k + c;
+            r[i] = (u32)t;
+            c = t >> 32;
+        }
+    } else {
+        zero(r);
+        mul_row<0>(r, a, k, 0);
+        mul_row<1>(r, a, k, 0);
     }
 }
 
@@ -312,32 +436,21 @@ struct QuotEst {
     }
 };
 
-// One step of Algorithm D on the window w[0..NB]: subtract qhat * bn, add
-// back once when qhat was one too large; returns the digit.
+// One step of Algorithm D on the window w[0..NB]: subtract qhat * b, add b
+// back once when qhat was one too large; returns the digit.  nb = 2^(32 NB) - b:
+// w - qhat * b = w + qhat * nb - qhat * 2^(32 NB), two carry chains of one wide
+// multiply-add per limb.
 template <int NB>
-UP_DI u32 knuth_step(u32 (&w)[NB + 1], const u32 (&bn)[NB], u32 qhat) {
-    u64 carry = 0;
-    i64 borrow = 0;
-#pragma unroll
-    for (int i = 0; i < NB; i++) {
-        const u64 p = (u64)qhat * bn[i] + carry;
-        carry = p >> 32;
-        const i64 t = (i64)w[i] - (i64)(u32)p + borrow;
-        w[i] = (u32)t;
-        borrow = t >> 32;  // 0 or -1
-    }
-    const i64 t = (i64)w[NB] - (i64)carry + borrow;
-    w[NB] = (u32)t;
-    if (t < 0) {
+UP_DI u32 knuth_step(u32 (&w)[NB + 1], const u32 (&nb)[NB], u32 qhat) {
+    mul_row<0>(w, nb, qhat, 0);
+    mul_row<1>(w, nb, qhat, 0);
+    w[NB] -= qhat;
+    if ((int)w[NB] < 0) {
         qhat--;
-        u64 c = 0;
+        w[0] = sub_cc(w[0], nb[0]);
 #pragma unroll
-        for (int i = 0; i < NB; i++) {
-            c += (u64)w[i] + bn[i];
-            w[i] = (u32)c;
-            c >>= 32;
-        }
-        w[NB] += (u32)c;
+        for (int i = 1; i < NB; i++) w[i] = subc_cc(w[i], nb[i]);
+        w[NB] = subc(w[NB], 0xffffffffu);  // + 2^(32 NB) - borrow
     }
     return qhat;
 }
@@ -411,6 +524,7 @@ UP_DI void divmod_norm(u32 (&q)[NX], u32 (&rn)[NB], u32 (&bn)[NB], u32& s, const
     }
     QuotEst est;
     est.init(bn[NB - 1], bn[NB - 2]);
+    negate(bn);  // the steps take 2^(32 NB) - bn
     // digits j = jmax .. 0 with jmax = nx - nb; the window of digit j is un[j .. j+NB]
     const int jmax = (int)((bitlen(x) + 31u) >> 5) - (int)((bl + 31u) >> 5);
 #pragma unroll
@@ -418,6 +532,7 @@ UP_DI void divmod_norm(u32 (&q)[NX], u32 (&rn)[NB], u32 (&bn)[NB], u32& s, const
     if (jmax < 0) {  // x < b: the remainder is x itself
 #pragma unroll
         for (int i = 0; i < NB; i++) rn[i] = un[i];
+        negate(bn);
         return;
     }
     if constexpr (!kUnroll && NB <= 64) {
@@ -466,6 +581,7 @@ UP_DI void divmod_norm(u32 (&q)[NX], u32 (&rn)[NB], u32 (&bn)[NB], u32& s, const
         }
 #pragma unroll
         for (int i = 0; i < NB; i++) rn[i] = w[i];
+        negate(bn);
         return;
     }
     // Static window positions: digit j uses un[j .. j+NB], j <= jmax <= NX - 1.
@@ -483,6 +599,7 @@ UP_DI void divmod_norm(u32 (&q)[NX], u32 (&rn)[NB], u32 (&bn)[NB], u32& s, const
     // the remainder (< bn) sits in un[0..NB)
 #pragma unroll
     for (int i = 0; i < NB; i++) rn[i] = un[i];
+    negate(bn);
     }
 }
 
@@ -522,13 +639,13 @@ UP_DI void div_small_quotient(u32 (&q)[NX], bool& up, const u32 (&x)[NX], const 
         add(rr, rr, b);
         u32 one[1] = {1u};
         sub(qv, qv, one);
-    } else if (cmp(rr, b) >= 0) {  // one too small
+    } else if (!less(rr, b)) {  // one too small
         sub(rr, rr, b);
         add_small(qv, 1u);
     }
     u32 dbl[NB + 2];
     add(dbl, rr, rr);
-    up = cmp(dbl, b) >= 0;
+    up = !less(dbl, b);
 #pragma unroll
     for (int i = 0; i < NX; i++) q[i] = i < 2 ? qv[i < 2 ? i : 0] : 0u;
 }
@@ -606,7 +723,7 @@ UP_DI u32 div_round(u32 (&r)[NR], u32& sr, const u32 (&a)[NA], u32 sa, const u32
         divmod_norm(q, rn, bn, s, x, b);
         u32 dbl[NB + 1];
         add(dbl, rn, rn);
-        up = cmp(dbl, bn) >= 0;
+        up = !less(dbl, bn);
     }
     copy_ext(r, q);
     if (up) add_small(r, 1u);
@@ -790,11 +907,51 @@ UP_DI void ld_compact_global(const u8* __restrict__ p, u32 (&m)[N], u32& sign) {
     m[TOPL] &= (TOPB == 31) ? 0x7fffffffu : ((1u << TOPB) - 1u);
 }
 
-// A column value by how its memory may be read: 1 the words around it (a
-// padded tile), 2 whole words of the value's column only, 0 bytes.
+// A value of a shared-memory tile whose first value is 16-byte aligned: the
+// widest loads B allows from 16 bytes on (words at a stride of 8 or 16 words
+// meet in the same banks: a*b+c at p=76 spent its time there, with the stores
+// below 0.307 -> 0.220 ms on B200; of 8-byte values p=18 took 0.117 ms in
+// words, 0.122 ms in pairs).
+template <int B, int N>
+UP_DI void ld_compact_tile(const u8* p, u32 (&m)[N], u32& sign) {
+    static_assert(N * 4 >= B, "limbs too few for the compact width");
+    if constexpr (B % 4 != 0 || B < 16) {
+        ld_compact_words<B, N>(p, m, sign);
+    } else {
+        constexpr int TOPL = B / 4 - 1;
+        zero(m);
+        if constexpr (B % 16 == 0) {
+#pragma unroll
+            for (int i = 0; i < B / 16; i++) {
+                const uint4 v = ((const uint4*)p)[i];
+                m[4 * i] = v.x;
+                m[4 * i + 1] = v.y;
+                m[4 * i + 2] = v.z;
+                m[4 * i + 3] = v.w;
+            }
+        } else if constexpr (B % 8 == 0) {
+#pragma unroll
+            for (int i = 0; i < B / 8; i++) {
+                const uint2 v = ((const uint2*)p)[i];
+                m[2 * i] = v.x;
+                m[2 * i + 1] = v.y;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < B / 4; i++) m[i] = ((const u32*)p)[i];
+        }
+        sign = m[TOPL] >> 31;
+        m[TOPL] &= 0x7fffffffu;
+    }
+}
+
+// A column value by how its memory may be read: 3 a tile of 16-byte aligned
+// values, 1 the words around it (padded), 2 whole words of the value's column
+// only, 0 bytes.
 template <int B, int N>
 UP_DI void ld_compact(const u8* p, int words, u32 (&m)[N], u32& sign) {
-    if (words == 1) ld_compact_words<B, N>(p, m, sign);
+    if (words == 3) ld_compact_tile<B, N>(p, m, sign);
+    else if (words == 1) ld_compact_words<B, N>(p, m, sign);
     else if (words == 2) ld_compact_global<B, N>(p, m, sign);
     else ld_compact_bytes<B, N>(p, m, sign);
 }
@@ -828,16 +985,28 @@ UP_DI u32 st_compact_bytes(u8* p, const u32 (&m)[N], u32 sign) {
     return compact_overflow<B>(m);
 }
 
-// Same, 4-byte aligned p and B % 4 == 0: word stores.
+// Same, p a value of a 16-byte aligned tile and B % 4 == 0: word stores.
 template <int B, int N>
 UP_DI u32 st_compact_words(u8* p, const u32 (&m)[N], u32 sign) {
     static_assert(B % 4 == 0, "word store needs B % 4 == 0");
-    u32* w = (u32*)p;
+    constexpr int W = B / 4;
+    u32 x[W];
 #pragma unroll
-    for (int i = 0; i < B / 4; i++) {
-        u32 v = at(m, i);
-        if (i == B / 4 - 1) v |= sign << 31;
-        w[i] = v;
+    for (int i = 0; i < W; i++) x[i] = at(m, i) | (i == W - 1 ? sign << 31 : 0u);
+#ifndef UP_HOST_TEST
+    // the widest stores B allows from 32 bytes on (p: a value of a 16-byte
+    // aligned tile)
+    if constexpr (W % 4 == 0 && W >= 8) {
+#pragma unroll
+        for (int i = 0; i < W; i += 4) ((uint4*)p)[i / 4] = make_uint4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+    } else if constexpr (W % 2 == 0 && W >= 8) {
+#pragma unroll
+        for (int i = 0; i < W; i += 2) ((uint2*)p)[i / 2] = make_uint2(x[i], x[i + 1]);
+    } else
+#endif
+    {
+#pragma unroll
+        for (int i = 0; i < W; i++) ((u32*)p)[i] = x[i];
     }
     return compact_overflow<B>(m);
 }
@@ -1710,11 +1879,29 @@ UP_DI const u8* col_ptr(const KCol& c, i64 row) {
 // ------------------------------------------------- tile staging helpers
 // Cooperative copy of n bytes global -> shared.  16-byte vectors when both
 // ends allow it, bytes otherwise.
+// Eight vectors of a thread are in flight at a time (a load and its store in
+// turn wait for the memory once per vector).
+UP_DI void tile_copy_vec(uint4* __restrict__ d, const uint4* __restrict__ s, int n) {
+    int i = threadIdx.x;
+    const int T = blockDim.x;
+    for (; i + 7 * T < n; i += 8 * T) {
+        uint4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = s[i + k * T];
+#pragma unroll
+        for (int k = 0; k < 8; k++) d[i + k * T] = v[k];
+    }
+    for (; i + T < n; i += 2 * T) {
+        const uint4 v0 = s[i], v1 = s[i + T];
+        d[i] = v0;
+        d[i + T] = v1;
+    }
+    if (i < n) d[i] = s[i];
+}
+
 UP_DI void tile_copy_in(u8* __restrict__ dst, const u8* __restrict__ src, int n, bool vec_ok) {
     if (vec_ok && (n & 15) == 0) {
-        const uint4* s = (const uint4*)src;
-        uint4* d = (uint4*)dst;
-        for (int i = threadIdx.x; i < (n >> 4); i += blockDim.x) d[i] = s[i];
+        tile_copy_vec((uint4*)dst, (const uint4*)src, n >> 4);
     } else {
         for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
     }
@@ -1722,9 +1909,7 @@ UP_DI void tile_copy_in(u8* __restrict__ dst, const u8* __restrict__ src, int n,
 
 UP_DI void tile_copy_out(u8* __restrict__ dst, const u8* __restrict__ src, int n, bool vec_ok) {
     if (vec_ok && (n & 15) == 0) {
-        const uint4* s = (const uint4*)src;
-        uint4* d = (uint4*)dst;
-        for (int i = threadIdx.x; i < (n >> 4); i += blockDim.x) d[i] = s[i];
+        tile_copy_vec((uint4*)dst, (const uint4*)src, n >> 4);
     } else {
         for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
     }
@@ -1798,18 +1983,6 @@ template <int N, int M>
 UP_DI void to_twos(u32 (&t)[N], const u32 (&m)[M], u32 sign) {
     copy_ext(t, m);
     if (sign) negate(t);
-}
-
-// r += t modulo 2^(32N) (two's complement accumulate in registers).
-template <int N>
-UP_DI void add_twos(u32 (&r)[N], const u32 (&t)[N]) {
-    u64 c = 0;
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        c += (u64)r[i] + t[i];
-        r[i] = (u32)c;
-        c >>= 32;
-    }
 }
 
 template <int NACC, int N>
