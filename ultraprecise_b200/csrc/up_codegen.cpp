@@ -291,7 +291,7 @@ struct TEmitter {
     // words of a warp's scratch for a product (tc_words of the device header)
     int tc_words(int la, int lb, bool constant) const {
         const int aw = (16 + std::max(la + 20, T * K) + 3) / 4 * 4;
-        const int out = ((la + lb + 1) / 2 + 15) / 16 * 64;
+        const int out = ((la + lb + 1) / 2 + 15) / 16 * 144;
         return 32 / T * (aw + std::max(out, constant ? 0 : 4 * tc_copy(lb)));
     }
     // the shifted copies of a constant as tc_stage_b lays them out
@@ -743,7 +743,8 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         const int CT = 256;               // CTA threads
         const int G = CT / tpiT;          // values in flight per CTA
         R = 1024;
-        while (R > 16 && (long)R * row_bytes > 32 * 1024) R /= 2;
+        // tensor products run two CTAs per SM, each with room for larger tiles
+        while (R > 16 && (long)R * row_bytes > (te.scratch_words ? 60 : 32) * 1024) R /= 2;
         std::vector<int> off;
         for (int c : used) {
             off.push_back(smem);
@@ -760,7 +761,8 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         if (cmp_root)
             src << "    if (store && tpi_rank<" << tpiT << ">() == 0) out[0] = (u8)c" << root << ";\n";
         else
-            src << "    err |= tpi_st<" << tpiT << ", " << tpiK << ", " << BO << ">(out, v" << root << ", s" << root
+            src << "    err |= tpi_st" << (BO >= 4 && BO <= 4 * tpiT * tpiK - 4 ? "_words" : "") << "<" << tpiT << ", " << tpiK << ", " << BO
+                << ">(out, v" << root << ", s" << root
                 << ", store);\n";
         src << "    return err;\n}\n\n";
         // four CTAs per SM (at most 64 registers): measured on B200, p=600

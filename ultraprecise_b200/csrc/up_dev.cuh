@@ -1111,23 +1111,53 @@ UP_DI bool tpi_is_zero(const u32 (&a)[K]) {
     return tpi_ballot<T>(o != 0u) == 0u;
 }
 
+// x += cin at each thread's lowest limb and the carries between threads;
+// returns the carry out of the top thread.  c, all: the carry out of the
+// thread's own limbs and the AND of them.
+template <int T, int K>
+UP_DI bool tpi_carry_fix(u32 (&x)[K], bool c, u32 all) {
+    const u32 G = tpi_ballot<T>(c);
+    const u32 A = G | tpi_ballot<T>(all == kFull);
+    const u64 sum = (u64)A + G;
+    tpi_inc_local(x, (u32)((sum ^ A ^ G) >> tpi_rank<T>()) & 1u);
+    return ((sum >> T) & 1u) != 0u;
+}
+
 // Signed add with the sign rules of add_signed (equal magnitudes of opposite
-// sign give +0).
+// sign give +0): a + b, or a - b as a + ~b + 1, negated where no carry comes
+// out (a < b).
 template <int T, int K>
 UP_DI void tpi_add_signed(u32 (&r)[K], u32& sr, const u32 (&a)[K], u32 sa, const u32 (&b)[K], u32 sb) {
-    const int c = tpi_cmp<T, K>(a, b);
-    u32 x[K], y[K], sum[K], dif[K];
+    const bool low = tpi_rank<T>() == 0;
+    const bool same = sa == sb;
+    const u32 x = same ? 0u : kFull;
+    const u32 one = low ? x : 0u;  // the carry in of a subtraction
+    u32 s[K], all = kFull, any = 0u;
+    add_cc(one, one);
+#pragma unroll
+    for (int i = 0; i < K; i++) s[i] = addc_cc(a[i], b[i] ^ x);
+    const u32 c = addc(0u, 0u);
+#pragma unroll
+    for (int i = 0; i < K; i++) all &= s[i];
+    const bool neg = !tpi_carry_fix<T>(s, c != 0u, all) && !same;
+    if (__any_sync(kFull, neg)) {
+        const u32 n = neg ? kFull : 0u, up = low ? n : 0u;
+        add_cc(up, up);
+#pragma unroll
+        for (int i = 0; i < K; i++) s[i] = addc_cc(s[i] ^ n, 0u);
+        const u32 c2 = addc(0u, 0u);
+        all = kFull;
+#pragma unroll
+        for (int i = 0; i < K; i++) all &= s[i];
+        tpi_carry_fix<T>(s, c2 != 0u, all);
+    }
 #pragma unroll
     for (int i = 0; i < K; i++) {
-        x[i] = c >= 0 ? a[i] : b[i];
-        y[i] = c >= 0 ? b[i] : a[i];
+        r[i] = s[i];
+        any |= s[i];
     }
-    tpi_add<T, K>(sum, a, b);
-    tpi_sub<T, K>(dif, x, y);
-    const bool same = sa == sb;
-#pragma unroll
-    for (int i = 0; i < K; i++) r[i] = same ? sum[i] : dif[i];
-    sr = same ? sa : (c == 0 ? 0u : (c > 0 ? sa : sb));
+    const bool nz = tpi_ballot<T>(any != 0u) != 0u;
+    sr = same ? sa : (nz ? (neg ? sb : sa) : 0u);
 }
 
 // Signed comparison with the rules of compare (-0 < +0).
@@ -1290,11 +1320,10 @@ UP_DI void tpi_mul_const(u32 (&r)[K], const u32 (&a)[K], const u32 (&p)[NP]) {
 // is below 255^2 * 4 * LB < 2^31).  The step of 8 bytes per row makes every A
 // fragment word one byte-swapped limb of a at index 2u - (l + 7 - 8) / 4, so a
 // lane's fragments of all tiles and steps are one sequence X(j) of words; B
-// fragments come from four copies of b shifted by 0..3 bytes.  The eight
-// positions of a row u are spread over a quad: after exchanging halves every
-// lane holds one limb's sum (below 2^51) per tile.  The limb sums go through
-// the warp's scratch back to the spread layout, where carries resolve as in
-// tpi_add.  The warp's 32 / T values run one after the other.
+// fragments come from four copies of b shifted by 0..3 bytes.  The position
+// sums go through the warp's scratch back to the spread layout, where a
+// thread adds four positions per limb and carries resolve as in tpi_add.  The
+// warp's 32 / T values run one after the other.
 // Against the window product: 32 limb steps of shuffles and a wide multiply
 // each become a few tensor instructions.
 __host__ __device__ constexpr int tc_steps(int lb) { return (4 * lb + 7 + 31) / 32; }
@@ -1304,7 +1333,7 @@ __host__ __device__ constexpr int tc_copy(int lb) { return (8 * tc_steps(lb) + 4
 __host__ __device__ constexpr int tc_tiles(int la, int lb) { return ((la + lb + 1) / 2 + 15) / 16; }
 __host__ __device__ constexpr int tc_a_words(int t, int k, int la) { return (16 + (la + 20 > t * k ? la + 20 : t * k) + 3) / 4 * 4; }
 __host__ __device__ constexpr int tc_b_words(int la, int lb, bool constant) {
-    const int out = tc_tiles(la, lb) * 64, copies = constant ? 0 : 4 * tc_copy(lb);
+    const int out = tc_tiles(la, lb) * 144, copies = constant ? 0 : 4 * tc_copy(lb);
     return copies > out ? copies : out;
 }
 // scratch words of a warp for one product
@@ -1329,8 +1358,12 @@ UP_DI void tc_stage_a(u32* ws, const u32 (&a)[K]) {
     for (int i = 0; i < K; i += 4)
         *(uint4*)(A + 16 + g * K + i) = make_uint4(__byte_perm(a[i], 0u, 0x0123u), __byte_perm(a[i + 1], 0u, 0x0123u),
                                                    __byte_perm(a[i + 2], 0u, 0x0123u), __byte_perm(a[i + 3], 0u, 0x0123u));
-    for (int i = g; i < 16; i += T) A[i] = 0u;
-    for (int i = 16 + T * K + g; i < AW; i += T) A[i] = 0u;
+#pragma unroll
+    for (int i = 0; i < 16; i += T)
+        if (i + g < 16) A[i + g] = 0u;
+#pragma unroll
+    for (int i = 16 + T * K; i < AW; i += T)
+        if (i + g < AW) A[i + g] = 0u;
 }
 
 // The four shifted copies of every value of the warp: copy s, word 4 + w =
@@ -1356,15 +1389,17 @@ UP_DI void tc_stage_b(u32* ws, const u32 (&b)[K]) {
             B[s * CS + 2] = 0u;
             B[s * CS + 3] = s ? b[0] << (32 - 8 * s) : 0u;
         }
-        for (int i = 4 + (LB + 3) / 4 * 4 + g; i < CS; i += T) B[s * CS + i] = 0u;
+#pragma unroll
+        for (int i = 4 + (LB + 3) / 4 * 4; i < CS; i += T)
+            if (i + g < CS) B[s * CS + i + g] = 0u;
     }
 }
 
-// The product's limb sums of every value of the warp from staged operands;
+// The product's position sums of every value of the warp from staged operands;
 // with CONST the B words are those of a constant (bc, laid out like a copy
 // set, in device memory), the same for all values.
 template <int T, int K, int LA, int LB, bool CONST>
-UP_DI void tc_limb_sums(u32* ws, const u32* __restrict__ bc) {
+UP_DI void tc_position_sums(u32* ws, const u32* __restrict__ bc) {
     constexpr int AW = tc_a_words(T, K, LA), VW = AW + tc_b_words(LA, LB, CONST);
     constexpr int KS = tc_steps(LB), MT = tc_tiles(LA, LB), CS = tc_copy(LB);
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -1402,45 +1437,48 @@ UP_DI void tc_limb_sums(u32* ws, const u32* __restrict__ bc) {
                 }
             }
         __syncwarp();  // every lane has read this value's operands: the sums may take b's place
-        u64* o = (u64*)B;
+        // position p at word p + 4 * (p / 32): lanes of tc_collect read 32
+        // positions (K = 8) each, from different banks
 #pragma unroll
         for (int m = 0; m < MT; m++) {
-            const u64 w0 = (u64)(u32)c[m][1] * 256u + (u32)c[m][0], w1 = (u64)(u32)c[m][3] * 256u + (u32)c[m][2];
-            const bool odd = t & 1;
-            const u64 send = odd ? w0 : w1, keep = odd ? w1 : w0;
-            const u64 recv = __shfl_xor_sync(kFull, send, 1);
-            const u64 lo = odd ? recv : keep, hi = odd ? keep : recv;
-            o[2 * (16 * m + (odd ? 8 : 0) + g) + (t >> 1)] = lo + (hi << 16);
+            int* o = (int*)B + 144 * m + 8 * g + 2 * t + 4 * (g >> 2);
+            *(int2*)o = make_int2(c[m][0], c[m][1]);
+            *(int2*)(o + 72) = make_int2(c[m][2], c[m][3]);
         }
     }
     __syncwarp();
 }
 
-// The limb sums back in the spread layout, carries resolved (low T*K limbs).
+// The position sums as limbs in the spread layout, carries resolved (low T*K limbs).
 template <int T, int K, int LA, int LB, bool CONST>
 UP_DI void tc_collect(u32 (&r)[K], const u32* ws) {
     constexpr int AW = tc_a_words(T, K, LA), VW = AW + tc_b_words(LA, LB, CONST), NL = tc_tiles(LA, LB) * 32;
     const int g = tpi_rank<T>();
-    const u64* o = (const u64*)(ws + (int)((threadIdx.x & 31u) / T) * VW + AW);
+    const u32* o = ws + (int)((threadIdx.x & 31u) / T) * VW + AW;
     u64 c = 0;
 #pragma unroll
     for (int i = 0; i < K; i++) {
-        if (g * K + i < NL) c += o[g * K + i];
+        const int l = g * K + i;
+        if (l < NL) {
+            const uint4 q = *(const uint4*)(o + 4 * l + 4 * (l >> 3));
+            c += q.x;
+            c += (u64)q.y * 0x100u;
+            c += (u64)q.z * 0x10000u;
+            c += (u64)q.w * 0x1000000u;
+        }
         r[i] = (u32)c;
         c >>= 32;
     }
     u32 in = __shfl_up_sync(kFull, (u32)c, 1, T);  // below 2^20
     if (g == 0) in = 0u;
-    c = in;
     u32 all = kFull;
+    r[0] = add_cc(r[0], in);
 #pragma unroll
-    for (int i = 0; i < K; i++) {
-        c += r[i];
-        r[i] = (u32)c;
-        c >>= 32;
-        all &= r[i];
-    }
-    tpi_inc_local(r, tpi_carry_in<T>(c != 0, all == kFull));
+    for (int i = 1; i < K; i++) r[i] = addc_cc(r[i], 0u);
+    const u32 out = addc(0u, 0u);
+#pragma unroll
+    for (int i = 0; i < K; i++) all &= r[i];
+    tpi_carry_fix<T>(r, out != 0u, all);
     __syncwarp();  // the scratch is free again
 }
 
@@ -1452,7 +1490,7 @@ UP_DI void tpi_mul(u32 (&r)[K], const u32 (&a)[K], const u32 (&b)[K], u32* ws) {
     tc_stage_a<T, K, LA, VW>(ws, a);
     tc_stage_b<T, K, LB, VW, AW>(ws, b);
     __syncwarp();
-    tc_limb_sums<T, K, LA, LB, false>(ws, nullptr);
+    tc_position_sums<T, K, LA, LB, false>(ws, nullptr);
     tc_collect<T, K, LA, LB, false>(r, ws);
 }
 
@@ -1463,7 +1501,7 @@ UP_DI void tpi_mul_const(u32 (&r)[K], const u32 (&a)[K], const u32* __restrict__
     constexpr int VW = tc_a_words(T, K, LA) + tc_b_words(LA, NP, true);
     tc_stage_a<T, K, LA, VW>(ws, a);
     __syncwarp();
-    tc_limb_sums<T, K, LA, NP, true>(ws, pc);
+    tc_position_sums<T, K, LA, NP, true>(ws, pc);
     tc_collect<T, K, LA, NP, true>(r, ws);
 }
 
@@ -1805,11 +1843,11 @@ UP_DI void tpi_ld_words(const u8* __restrict__ p, u32 (&x)[K], u32& sign) {
     const u32* w = (const u32*)(p - off);
     const u32 sh = off * 8u;
     constexpr int W = (B + 3) / 4;  // limbs holding bytes of the value
+    u32 y[K + 1];
 #pragma unroll
-    for (int i = 0; i < K; i++) {
-        const int L = g * K + i;
-        x[i] = L < W ? __funnelshift_r(w[L], w[L + 1], sh) : 0u;
-    }
+    for (int i = 0; i <= K; i++) y[i] = g * K + i <= W ? w[g * K + i] : 0u;
+#pragma unroll
+    for (int i = 0; i < K; i++) x[i] = g * K + i < W ? __funnelshift_r(y[i], y[i + 1], sh) : 0u;
     sign = (u32)(p[B - 1] >> 7);
     constexpr int TOPL = (B - 1) / 4;
     constexpr int TOPB = ((B - 1) % 4) * 8 + 7;  // the sign bit; the bits above it belong to the next value
@@ -1847,6 +1885,50 @@ UP_DI u32 tpi_st(u8* __restrict__ p, const u32 (&x)[K], u32 sign, bool store) {
             for (int o = 4 * T * K + g; o < B; o += T) p[o] = (u8)(o == B - 1 ? sign << 7 : 0u);
     }
     return tpi_ballot<T>(over) ? ERR_OVERFLOW : 0u;
+}
+
+// tpi_st into a shared-memory tile, at any alignment: aligned words of the
+// value's bytes from two neighbouring limbs each, bytes only in the first and
+// last words (32 byte stores per thread otherwise).  B at most 4*T*K - 4.
+template <int T, int K, int B>
+UP_DI u32 tpi_st_words(u8* __restrict__ p, const u32 (&x)[K], u32 sign, bool store) {
+    static_assert(B <= 4 * T * K - 4, "the last word belongs to a thread");
+    constexpr int TOPL = (B - 1) / 4;
+    constexpr int TOPB = ((B - 1) % 4) * 8 + 7;
+    constexpr u32 KEEP = TOPB == 31 ? 0x7fffffffu : (1u << TOPB) - 1u;
+    const int g = tpi_rank<T>();
+    u32 over = 0u, y[K];
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        const int l = g * K + i;
+        y[i] = x[i];
+        if (l > TOPL) over |= x[i];
+        if (l == TOPL) {
+            over |= x[i] & ~KEEP;
+            y[i] |= sign << TOPB;
+        }
+    }
+    u32 below = __shfl_up_sync(kFull, y[K - 1], 1, T);
+    if (g == 0) below = 0u;
+    if (store) {
+        const int off = (int)((unsigned long long)p & 3u), last = (B + off) >> 2;  // words 0 (1) .. last-1 are whole
+        u8* base = p - off;
+        u32 tail = 0u;
+#pragma unroll
+        for (int i = 0; i < K; i++) {
+            const int m = g * K + i;
+            const u32 v = __funnelshift_l(i ? y[i ? i - 1 : 0] : below, y[i], 8u * (u32)off);
+            if (i == 0 && g == 0 && off) {
+                for (int k = off; k < 4; k++) base[k] = (u8)(v >> (8 * k));
+            } else if (m < last) {
+                *(u32*)(base + 4 * m) = v;
+            }
+            if (m == last) tail = v;
+        }
+        if (last / K == g)
+            for (int k = 0; k < ((B + off) & 3); k++) base[4 * last + k] = (u8)(tail >> (8 * k));
+    }
+    return tpi_ballot<T>(over != 0u) ? ERR_OVERFLOW : 0u;
 }
 
 #endif  // UP_HOST_TEST
