@@ -113,6 +113,63 @@ static long check_sums(long n) {
     return bad;
 }
 
+// x = q*b + r with r < b and quotients around every bound of
+// div_small_quotient (2^47, 2^79: above it the function declines)
+template <int NX, int NB>
+static long check_quotient(long n) {
+    long bad = 0, ran = 0;
+    for (long c = 0; c < n; c++) {
+        u32 b[NB], r[NB], q[NX] = {0}, x[NX], got[NX];
+        gen(b);
+        for (int i = 2 + (int)(rnd() % (NB - 1)); i < NB; i++) b[i] = 0u;
+        if (NB > 1 && rnd() % 2) b[1] |= 1u;
+        bool wide = false;
+        for (int i = 1; i < NB; i++) wide |= b[i] != 0u;
+        if (!wide) continue;
+        const int bits = (int)(rnd() % 83);  // of the quotient
+        for (int i = 0; i < NX; i++) {
+            const int left = bits - 32 * i;
+            const u32 v = rnd() % 3 == 0 ? 0xffffffffu : (rnd() % 2 ? rnd() : 0u);
+            q[i] = left <= 0 ? 0u : (left >= 32 ? v : v & ((1u << left) - 1u));
+        }
+        if (rnd() % 4 == 0)
+            for (int i = 0; i < NX; i++) q[i] = i == bits / 32 ? 1u << (bits % 32) : 0u;
+        const int rm = rnd() % 4;  // 0, b - 1, b / 2 and neighbours
+        for (int i = 0; i < NB; i++)
+            r[i] = rm == 0 ? 0u : (rm == 1 ? b[i] : (b[i] >> 1) | (i + 1 < NB ? b[i + 1 < NB ? i + 1 : 0] << 31 : 0u));
+        if (rm == 1) {
+            u32 one[1] = {1u};
+            sub(r, r, one);
+        }
+        if (rm == 3) {
+            u32 one[1] = {1u};
+            add(r, r, one);
+            if (!less(r, b)) continue;
+        }
+        u32 full[NX + NB + 1];
+        mul(full, q, b);
+        add(full, full, r);
+        bool fits = true;
+        for (int i = NX; i < NX + NB + 1; i++) fits &= full[i] == 0u;
+        if (!fits) continue;
+        for (int i = 0; i < NX; i++) x[i] = full[i];
+        bool up = false;
+        ran++;
+        if (!div_small_quotient(got, up, x, b)) {
+            bad += bits < 78;
+            continue;
+        }
+        u32 dbl[NB + 1];
+        add(dbl, r, r);
+        bool ok = up == !less(dbl, b);
+        for (int i = 0; i < NX; i++) ok &= got[i] == q[i];
+        if (!ok && bad < 3) std::printf("quotient<%d,%d> of %d bits, rm %d\n", NX, NB, bits, rm);
+        bad += !ok;
+    }
+    std::printf("quotient<%d,%d> %ld %ld\n", NX, NB, ran, bad);
+    return bad;
+}
+
 int main(int argc, char** argv) {
     const long n = argc > 1 ? std::atol(argv[1]) : 20000;
     long bad = 0;
@@ -123,5 +180,7 @@ int main(int argc, char** argv) {
     bad += check_mul<3, 4, 4>(n) + check_mul<7, 8, 8>(n) + check_mul<20, 16, 16>(n / 8);  // low limbs only
     bad += check_sums<1, 1, 1>(n) + check_sums<4, 4, 3>(n) + check_sums<5, 5, 5>(n) + check_sums<6, 4, 5>(n);
     bad += check_sums<9, 8, 3>(n) + check_sums<33, 32, 32>(n / 4);
+    bad += check_quotient<3, 2>(n) + check_quotient<5, 2>(n) + check_quotient<6, 4>(n) + check_quotient<7, 4>(n);
+    bad += check_quotient<8, 4>(n) + check_quotient<7, 5>(n) + check_quotient<6, 6>(n);
     return bad ? 1 : 0;
 }
