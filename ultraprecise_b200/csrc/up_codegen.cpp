@@ -278,9 +278,10 @@ struct TEmitter {
     bool tensor = false;       // wide products on the tensor cores, through a warp's scratch `ws`
     int scratch_words = 0;     // of a warp, for the products emitted so far
 
-    // Operand limbs from which a product goes to the tensor cores: the window
-    // product costs a step of shuffles per limb of the shorter operand, the
-    // tensor one a nearly fixed number of instructions.
+    // Operand limbs from which a product goes to the tensor cores: six limbs and
+    // the seven bytes of shift fill one 32-byte step of the fragments; the
+    // window product costs a step of shuffles per limb, the tensor one a nearly
+    // fixed number of instructions per step.
     static constexpr int kTensorMinLimbs = 6;
     bool on_tensor(int lb) const { return tensor && !out_of_line && K % 4 == 0 && K <= 16 && lb >= kTensorMinLimbs; }
     static int tc_steps(int lb) { return (4 * lb + 7 + 31) / 32; }
@@ -470,9 +471,10 @@ struct TEmitter {
     }
 };
 
-// Automatic cooperative evaluation starts at this width: measured on B200,
-// a*b+c at p=600 (127 limbs) runs 1.26x faster cooperatively, while at p=300
-// (64 limbs) and p=150 (32 limbs) one thread per value is faster.
+// Automatic cooperative evaluation starts at this width: measured on B200, with
+// one thread per value and cooperatively, a*b+c at p=600 (127 limbs, 512K rows)
+// 1.14 and 0.73 ms, at p=450 (95 limbs) 0.58 and 0.63 ms, at p=300 (64 limbs, 1M
+// rows) 0.48 and 0.66 ms.
 constexpr int kCoopMinLimbs = 96;
 
 // Widest limb count a cooperative evaluation of the expression needs (every
@@ -780,7 +782,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         for (size_t i = 0; i < used.size(); i++) {
             const int cc = used[i];
             const int B = compact_bytes(cols[cc].precision);
-            src << "        tile_copy_in(sm + " << off[i] << ", a.col[" << cc << "].data + row0 * " << B << ", nr * " << B
+            src << "        tile_copy_in<true>(sm + " << off[i] << ", a.col[" << cc << "].data + row0 * " << B << ", nr * " << B
                 << ", a.vec_ok != 0);\n";
         }
         src << "        __syncthreads();\n";
@@ -795,7 +797,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
             << ws_words << ");\n";
         src << "            if (valid) err |= e;\n        }\n";
         src << "        __syncthreads();\n";
-        src << "        tile_copy_out(a.out + row0 * " << BO << ", sm + " << off_out << ", nr * " << BO
+        src << "        tile_copy_out<true>(a.out + row0 * " << BO << ", sm + " << off_out << ", nr * " << BO
             << ", a.vec_ok != 0);\n";
         src << "        __syncthreads();\n    }\n";
         T = CT;
@@ -917,7 +919,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         for (size_t i = 0; i < used.size(); i++) {
             int c = used[i];
             int B = compact_bytes(cols[c].precision);
-            src << "        tile_copy_in(sm + " << off[i] << ", a.col[" << c << "].data + row0 * " << B << ", nr * "
+            src << "        tile_copy_in<true>(sm + " << off[i] << ", a.col[" << c << "].data + row0 * " << B << ", nr * "
                 << B << ", a.vec_ok != 0);\n";
         }
         src << "        __syncthreads();\n";
@@ -929,7 +931,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         }
         src << "sm + " << off_out << " + r * " << BO << ", 3);\n";
         src << "        __syncthreads();\n";
-        src << "        tile_copy_out(a.out + row0 * " << BO << ", sm + " << off_out << ", nr * " << BO
+        src << "        tile_copy_out<true>(a.out + row0 * " << BO << ", sm + " << off_out << ", nr * " << BO
             << ", a.vec_ok != 0);\n";
         src << "        __syncthreads();\n    }\n";
     }
@@ -964,7 +966,7 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         for (size_t i = 0; i < used.size(); i++) {
             const int c = used[i];
             const int B = compact_bytes(cols[c].precision);
-            src << "        tile_copy_in(sm + " << moff[i] << ", q.col[" << c << "].data + row0 * " << B << ", nr * " << B
+            src << "        tile_copy_in<true>(sm + " << moff[i] << ", q.col[" << c << "].data + row0 * " << B << ", nr * " << B
                 << ", q.vec_ok != 0);\n";
         }
         src << "        __syncthreads();\n        u32 err = 0u;\n";

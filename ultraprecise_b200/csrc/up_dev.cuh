@@ -2001,37 +2001,39 @@ UP_DI const u8* col_ptr(const KCol& c, i64 row) {
 // ------------------------------------------------- tile staging helpers
 // Cooperative copy of n bytes global -> shared.  16-byte vectors when both
 // ends allow it, bytes otherwise.
-// Eight vectors of a thread are in flight at a time (a load and its store in
-// turn wait for the memory once per vector).
+// WIDE: eight vectors of a thread are in flight at a time, for the kernels that
+// stage whole tiles this way (a load and its store in turn wait for the memory
+// once per vector).  The bulk-copy kernels only copy their last tile here and
+// keep the short loop (its registers cost a*b+c at p=18 2 %).
+template <bool WIDE = false>
 UP_DI void tile_copy_vec(uint4* __restrict__ d, const uint4* __restrict__ s, int n) {
     int i = threadIdx.x;
-    const int T = blockDim.x;
-    for (; i + 7 * T < n; i += 8 * T) {
-        uint4 v[8];
+    if constexpr (WIDE) {
+        const int T = blockDim.x;
+        for (; i + 7 * T < n; i += 8 * T) {
+            uint4 v[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = s[i + k * T];
+            for (int k = 0; k < 8; k++) v[k] = s[i + k * T];
 #pragma unroll
-        for (int k = 0; k < 8; k++) d[i + k * T] = v[k];
+            for (int k = 0; k < 8; k++) d[i + k * T] = v[k];
+        }
     }
-    for (; i + T < n; i += 2 * T) {
-        const uint4 v0 = s[i], v1 = s[i + T];
-        d[i] = v0;
-        d[i + T] = v1;
-    }
-    if (i < n) d[i] = s[i];
+    for (; i < n; i += blockDim.x) d[i] = s[i];
 }
 
+template <bool WIDE = false>
 UP_DI void tile_copy_in(u8* __restrict__ dst, const u8* __restrict__ src, int n, bool vec_ok) {
     if (vec_ok && (n & 15) == 0) {
-        tile_copy_vec((uint4*)dst, (const uint4*)src, n >> 4);
+        tile_copy_vec<WIDE>((uint4*)dst, (const uint4*)src, n >> 4);
     } else {
         for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
     }
 }
 
+template <bool WIDE = false>
 UP_DI void tile_copy_out(u8* __restrict__ dst, const u8* __restrict__ src, int n, bool vec_ok) {
     if (vec_ok && (n & 15) == 0) {
-        tile_copy_vec((uint4*)dst, (const uint4*)src, n >> 4);
+        tile_copy_vec<WIDE>((uint4*)dst, (const uint4*)src, n >> 4);
     } else {
         for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
     }
