@@ -2017,6 +2017,11 @@ UP_DI void tile_copy_vec(uint4* __restrict__ d, const uint4* __restrict__ s, int
 #pragma unroll
             for (int k = 0; k < 8; k++) d[i + k * T] = v[k];
         }
+        for (; i + T < n; i += 2 * T) {
+            const uint4 v0 = s[i], v1 = s[i + T];
+            d[i] = v0;
+            d[i + T] = v1;
+        }
     }
     for (; i < n; i += blockDim.x) d[i] = s[i];
 }
