@@ -72,6 +72,11 @@ up_status up_util_auto_tpv(const up_expr_node* nodes, int32_t n_nodes, int32_t r
 int64_t up_util_expr_source(const up_expr_node* nodes, int32_t n_nodes, int32_t root, const up_col_type* cols,
                             int32_t n_cols, const up_compile_opts* opts, char* buf, int64_t cap);
 
+/* The same for a fused query module (up_query_compile's arguments). */
+int64_t up_util_query_source(const up_expr_node* nodes, int32_t n_nodes, const up_col_type* cols, int32_t n_cols,
+                             const up_query_agg* aggs, int32_t n_aggs, const up_compile_opts* opts, char* buf,
+                             int64_t cap);
+
 /* NVRTC-compile a batch module into the cubin cache (no GPU): tpv_of gives
  * each task's threads per value, NULL the automatic choice (tpv_policy 0). */
 struct up_batch_task;

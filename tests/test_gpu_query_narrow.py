@@ -84,3 +84,25 @@ def test_register_sums_over_many_tiles():
     want = [int((a.long() * b.long())[gid == g].sum().item()) for g in range(3)]
     got = [d["mag"] for d in codec.decode_agg(_raw(outs[0]), 3)]
     assert got == want
+
+
+@pytest.mark.parametrize("groups", [3, 7])
+def test_columns_met_in_any_order(groups):
+    """Expressions that meet their columns out of order or leave some out,
+    columns of different precisions and scales, narrow and wide rows."""
+    a, b, c, d = (E.col(i) for i in range(4))
+    types = [(15, 2), (4, 1), (9, 4), (18, 0)]
+    rows = 5003
+    for exprs in ([b - a], [c * (E.dec("1.00") - a) + b], [c, c - a], [d * b, b - d], [d - c, b + a]):
+        rng = random.Random(groups)
+        aggs = [(abi.UP_AGG_SUM, i) for i in range(len(exprs))] + [(abi.UP_AGG_AVG, 0), (abi.UP_AGG_COUNT, 0)]
+        q = runtime.compile_query(exprs, aggs, [E.ColType(p, s) for p, s in types])
+        raws = [_column(rows, p, rng, 0.1) for p, _ in types]
+        cols = [runtime.DeviceColumn.from_host(r, p, s) for r, (p, s) in zip(raws, types)]
+        gid = torch.tensor([rng.randrange(groups) for _ in range(rows)], dtype=torch.int32, device="cuda")
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        outs = q.launch(cols, gid, groups, err=err)
+        exp = oracle.query(q.built, q.aggs, raws, _raw(gid), rows, groups, threads=8)
+        assert int(err.item()) == 0
+        for k, (o, e) in enumerate(zip(outs, exp)):
+            assert _raw(o) == e, f"aggregate {k}"

@@ -790,17 +790,29 @@ up_status up_util_auto_tpv(const up_expr_node* nodes, int32_t n_nodes, int32_t r
     return UP_OK;
 }
 
+static int64_t copy_source(const std::string& source, char* buf, int64_t cap) {
+    const int64_t n = (int64_t)source.size();
+    if (buf && cap > 0) {
+        const int64_t k = std::min(n, cap - 1);
+        memcpy(buf, source.data(), (size_t)k);
+        buf[k] = '\0';
+    }
+    return n;
+}
+
 int64_t up_util_expr_source(const up_expr_node* nodes, int32_t n_nodes, int32_t root, const up_col_type* cols,
                             int32_t n_cols, const up_compile_opts* opts, char* buf, int64_t cap) {
     GeneratedModule gen;
     if (generate_expr_module(nodes, n_nodes, root, cols, n_cols, opts, gen) != UP_OK) return -1;
-    const int64_t n = (int64_t)gen.source.size();
-    if (buf && cap > 0) {
-        const int64_t k = std::min(n, cap - 1);
-        memcpy(buf, gen.source.data(), (size_t)k);
-        buf[k] = '\0';
-    }
-    return n;
+    return copy_source(gen.source, buf, cap);
+}
+
+int64_t up_util_query_source(const up_expr_node* nodes, int32_t n_nodes, const up_col_type* cols, int32_t n_cols,
+                             const up_query_agg* aggs, int32_t n_aggs, const up_compile_opts* opts, char* buf,
+                             int64_t cap) {
+    GeneratedModule gen;
+    if (generate_query_module(nodes, n_nodes, cols, n_cols, aggs, n_aggs, opts, gen) != UP_OK) return -1;
+    return copy_source(gen.source, buf, cap);
 }
 
 up_status up_device_query(int32_t device, up_device_info* info) {

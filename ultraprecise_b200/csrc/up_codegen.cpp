@@ -1069,7 +1069,7 @@ struct NarrowEmitter {
     int col_bits = kSumCols;
     std::ostringstream body;
     std::vector<int> eb;  // bound of every node in bits
-    std::vector<int> roots, cols;
+    std::vector<int> roots;
     int tmp = 0;
     NarrowEmitter(const up_expr_node* n, const std::vector<NodeFacts>& facts) : nodes(n), f(facts) {}
 
@@ -1108,7 +1108,6 @@ struct NarrowEmitter {
             switch (nd.kind) {
                 case UP_NODE_COLUMN:
                     eb[k] = std::min(f[k].bits, col_bits);
-                    if (std::find(cols.begin(), cols.end(), nd.column) == cols.end()) cols.push_back(nd.column);
                     e = "x" + std::to_string(nd.column);
                     break;
                 case UP_NODE_CONST:
@@ -1158,9 +1157,11 @@ struct NarrowEmitter {
             for (int r : roots) check(v(r), eb[r], kSumBits);
         return true;
     }
-    std::string function() const {
+    // The parameters are the columns in `used` order, the order the kernels
+    // pass them in (an expression may meet its columns in any order).
+    std::string function(const std::vector<int>& used) const {
         std::string args, sets;
-        for (int c : cols) args += (args.empty() ? "i64 x" : ", i64 x") + std::to_string(c);
+        for (int c : used) args += (args.empty() ? "i64 x" : ", i64 x") + std::to_string(c);
         for (size_t i = 0; i < roots.size(); i++) {
             args += (args.empty() ? "i64& y" : ", i64& y") + std::to_string(i);
             sets += "    y" + std::to_string(i) + " = (i64)" + v(roots[i]) + ";\n";
@@ -1671,7 +1672,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
             out.q_smem_r = off_rbar + 16;
             out.q_threads_r = TR;
             out.q_tile_rows_r = RR;
-            src << nw.function();
+            src << nw.function(used);
             // KEYS: a row's key is matched against the present keys held in
             // registers (the inverse half of the key table), so no table lookup
             // happens per row; rows matching none are counted and flagged as a

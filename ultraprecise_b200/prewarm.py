@@ -33,6 +33,23 @@ def expr_source(root, cols, threads_per_value: int = 0) -> str:
     return buf.value.decode()
 
 
+def query_source(roots, cols, aggs, block_threads: int = 0) -> str:
+    """Generated CUDA source of a query module (CPU only); aggs as in
+    runtime.compile_query: (kind, index of its root)."""
+    lib = abi.load()
+    b = E.build(roots, cols)
+    E.derive_types(b)
+    qa = (abi.UpQueryAgg * len(aggs))(*[(k, b.roots[r]) for k, r in aggs])
+    opts = abi.UpCompileOpts(0, block_threads, 0)
+    args = (b.nodes, b.n_nodes, b.col_types, b.n_cols, qa, len(aggs), C.byref(opts))
+    n = lib.up_util_query_source(*args, None, 0)
+    if n < 0:
+        raise ValueError("query rejected")
+    buf = C.create_string_buffer(int(n) + 1)
+    lib.up_util_query_source(*args, buf, n + 1)
+    return buf.value.decode()
+
+
 def _compile(roots, cols, aggs=None):
     lib = abi.load()
     b = E.build(roots, cols)
