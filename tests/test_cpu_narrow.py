@@ -107,3 +107,56 @@ def test_columns_in_any_order(tmp_path):
             row = [rng.randint(-1000, 1000) for _ in types]
             taken += _check(lib, k, built, row)
         assert taken == 300
+
+
+def _edge(rng, bits):
+    """A value of at most `bits` bits, often next to a power of two."""
+    k = rng.randint(0, bits)
+    m = (1 << k) + rng.choice((-3, -1, 0, 0, 1, 3)) if rng.random() < 0.8 else rng.getrandbits(bits)
+    return rng.choice((-1, 1)) * min(abs(m), (1 << bits) - 1)
+
+
+def test_bounds_leave_both_ends_out(tmp_path):
+    """Two operands checked to 30 bits whose sum is -2^31, negated: a row whose
+    value an int does not hold is not taken."""
+    x0, x1, x2, x3, x4 = (E.col(i) for i in range(N_COLS))
+    types = [E.ColType(18, 0)] * N_COLS
+    b, c, a = x0 + x1, x2 + x3, (x0 + x2) + x4
+    roots = [a * b, a * c, -(b + c)]
+    lib = _host(tmp_path, [prewarm.query_source(roots, types, _sum_aggs(3))])
+    built = _built(roots, types)
+    h = 1 << 29
+    for x4v in (0, 1, 3, (1 << 30) - 1):
+        for s in (-1, 1):
+            for delta in (-1, 0, 1):
+                _check(lib, 0, built, [s * h, s * h, s * h, s * h + delta, x4v])
+    assert _check(lib, 0, built, [h, 1, -h, 5, 7])
+
+
+def _random_query(rng):
+    """Up to four sums over a pool of shared, sometimes negated nodes."""
+    types = [E.ColType(p, rng.randint(0, min(4, p))) for p in (rng.choice((4, 9, 12, 15, 18)) for _ in range(N_COLS))]
+    pool = [E.col(i) for i in range(N_COLS)] + [E.dec("1.00"), E.lit(-7)]
+    for _ in range(rng.randint(2, 7)):
+        x, y = rng.choice(pool), rng.choice(pool)
+        n = rng.choice((x + y, x - y, x * y))
+        pool.append(-n if rng.random() < 0.3 else n)
+    return pool[-rng.randint(1, 4):], types
+
+
+def test_random_nodes_at_their_bounds(tmp_path):
+    rng = random.Random(5)
+    queries, srcs = [], []
+    while len(queries) < 120:
+        roots, types = _random_query(rng)
+        src = prewarm.query_source(roots, types, _sum_aggs(len(roots)))
+        if "up_qnarrow" in src and "quad_value" in src:
+            queries.append((_built(roots, types), types, _col_bits(src)))
+            srcs.append(src)
+    lib = _host(tmp_path, srcs)
+    taken = 0
+    for k, (built, types, bits) in enumerate(queries):
+        for _ in range(400):
+            row = [_edge(rng, min(bits, 8 * codec.compact_bytes(t.precision) - 1)) for t in types]
+            taken += _check(lib, k, built, row)
+    assert taken > 5000

@@ -1076,9 +1076,11 @@ struct NarrowEmitter {
     static std::string v(int k) { return "n" + std::to_string(k); }
     static const char* type(int bits) { return bits <= 31 ? "int" : "i64"; }
     int sum_words(int i) const { return eb[roots[i]] <= kSumBits ? 2 : 3; }
+    // -2^limit < value < 2^limit: both ends left out, as every bound here means
+    // it (an int holds a value of 31 bits and its negation).
     void check(const std::string& name, int& bits, int limit) {
         if (bits <= limit) return;
-        body << "    ok = ok && ((u64)((i64)" << name << " + (1ll << " << limit << ")) >> " << limit + 1 << ") == 0ull;\n";
+        body << "    ok = ok && (u64)((i64)" << name << " + " << (1ll << limit) - 1 << "ll) < " << (2ull << limit) - 1 << "ull;\n";
         bits = limit;
     }
     // node a at scale sc: its name, its bound in `bits`
