@@ -1,7 +1,13 @@
 """Decimal text in and out: the Python restatement of the reference's parse
 (StringToDecimal + cast + ToCompactDecimal) and output image (GetDecimal),
 on hand-checked cases, and the round trip of the decimal string."""
+import os
 import random
+import re
+import shutil
+import subprocess
+
+import pytest
 
 from oracle import pyref
 from ultraprecise_b200 import codec
@@ -49,3 +55,31 @@ def test_round_trip():
             text = pyref.format_decimal(raw, s).encode()
             back, err = pyref.parse_decimal(text, B, s)
             assert err == 0 and back == raw, (p, s, v, text)
+
+
+def test_staged_fields_lie_in_the_staged_text(tmp_path):
+    """The rule by which the staged parser reads a field from shared memory,
+    compiled for the host: it never takes a field that starts or ends outside
+    the staged text, whatever the order of the offsets."""
+    if shutil.which("g++") is None:
+        pytest.skip("no g++")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    src = open(os.path.join(root, "ultraprecise_b200", "csrc", "up_text.cu")).read()
+    rule = re.search(r"constexpr bool staged_field\(.*?\n}\n", src, re.S).group(0)
+    assert "staged_field(a, b, lo, hi)" in src[src.index("k_parse_staged("):]
+    cpp, exe = str(tmp_path / "f.cpp"), str(tmp_path / "f")
+    with open(cpp, "w") as f:
+        f.write("#include <cstdint>\n" + rule + """
+int main() {
+    const int64_t v[] = {0, 1, 5, 6, 7, 1029, 1030, 1031, 5000, 9000, 9001, 1ll << 40};
+    int taken = 0;
+    for (int64_t lo : v) for (int64_t hi : v) for (int64_t a : v) for (int64_t b : v)
+        if (staged_field(a, b, lo, hi)) {
+            if (a < lo || a > hi || b < a || b > hi || b - a > 1024) return 1;
+            taken++;
+        }
+    return taken > 100 ? 0 : 2;
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-o", exe, cpp], check=True)
+    assert subprocess.run([exe]).returncode == 0

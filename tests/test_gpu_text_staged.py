@@ -85,3 +85,25 @@ def test_parse_fields_at_the_staged_edges(p, s):
     for _, e in want:
         exp_err |= e
     assert err == exp_err
+
+
+def test_parse_offsets_that_do_not_ascend():
+    """A field that ends before it starts reads nothing and stores 0; its
+    neighbours, and fields that overlap, are what they are alone."""
+    rng = random.Random(9)
+    text = "".join(rng.choice("0123456789") for _ in range(6000)).encode()
+    offsets = [rng.randrange(40)]
+    for r in range(700):
+        offsets.append(min(5900, offsets[-1] + rng.randrange(0, 12)) if rng.random() < 0.8 else rng.randrange(0, 5900))
+    offsets[128], offsets[256] = 3000, 3900  # two CTAs' ranges that ascend and fit, whatever is inside
+    p, s = 38, 0
+    B = codec.compact_bytes(p)
+    dev = torch.frombuffer(bytearray(text), dtype=torch.uint8).cuda()
+    got, err = runtime.parse_decimal(None, p, s, text=dev, offsets=torch.tensor(offsets, device="cuda"))
+    got = bytes(got.cpu().numpy().tobytes())
+    exp_err = 0
+    for r, (a, b) in enumerate(zip(offsets, offsets[1:])):
+        want, e = pyref.parse_decimal(text[a:max(a, b)], B, s)
+        assert got[r * B:(r + 1) * B] == want, (r, a, b)
+        exp_err |= e
+    assert err == exp_err

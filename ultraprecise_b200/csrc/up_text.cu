@@ -304,6 +304,13 @@ __device__ __forceinline__ bool parse_row_limbs(const u8* s, int n, int scale, u
     return ints + scale <= digits_of_limbs(N);
 }
 
+// Whether a field [a, b) lies in the staged text [lo, hi) and is short enough
+// for the limbs in registers.  Fields that end before they start (offsets that
+// do not ascend) read nothing: the general routine stores their 0.
+__host__ __device__ constexpr bool staged_field(int64_t a, int64_t b, int64_t lo, int64_t hi) {
+    return a >= lo && a <= b && b <= hi && b - a <= 1024;
+}
+
 // Bound by the instructions per character; a byte of text from global memory
 // per step and limbs in local memory waited on both.  The CTA's text (its
 // fields are consecutive) is staged in shared memory when it fits `cap`
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(kTextRows) k_parse_staged(const char* __restri
             const int64_t a = off[r0 + threadIdx.x], b = off[r0 + threadIdx.x + 1];
             u8* o = vals + threadIdx.x * B;
             bool done = false;
-            if (fits && a >= lo && b <= hi && b - a <= 1024) {
+            if (fits && staged_field(a, b, lo, hi)) {
                 u32 m[N], sign;
                 bool bad;
                 if (parse_row_limbs<N>(buf + (a - lo), (int)(b - a), scale, m, sign, bad)) {
