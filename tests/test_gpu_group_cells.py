@@ -1,5 +1,8 @@
 """Grouped aggregation in shared-memory cells and limb sums: group counts at
 the edges of the modes, signs, row counts that fold the cells midway."""
+import ctypes as C
+import random
+
 import numpy as np
 import pytest
 
@@ -69,3 +72,31 @@ def test_group_ids_out_of_range_are_flagged():
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     q.launch([runtime.DeviceColumn(t, p, 2) for t in cols], gid, groups, err=err)
     assert int(err.item()) == 4  # UP_ROWERR_DOMAIN
+
+
+@pytest.mark.parametrize("threads", [32, 96, 256])
+def test_cells_of_other_cta_sizes(threads):
+    """Query kernels compiled for other CTA sizes: replicated cells, one cell
+    per group, hashed cells."""
+    rng = random.Random(threads)
+    p, s, rows = 18, 4, 3001
+    b = E.derive_types(E.build([E.col(0) * E.col(1), E.col(0)], [E.ColType(p, s)] * 2))
+    aggs = [(abi.UP_AGG_SUM, b.roots[0]), (abi.UP_AGG_AVG, b.roots[1]), (abi.UP_AGG_COUNT, b.roots[1])]
+    qa = (abi.UpQueryAgg * 3)(*aggs)
+    lib, h = abi.load(), C.c_void_p()
+    opts = abi.UpCompileOpts(0, threads, 0)
+    abi.check(lib.up_query_compile(b.nodes, b.n_nodes, b.col_types, b.n_cols, qa, 3, C.byref(opts), C.byref(h)), "compile")
+    raws = [codec.encode([(rng.getrandbits(1), rng.randrange(10 ** p)) for _ in range(rows)], p) for _ in range(2)]
+    cols = [runtime.DeviceColumn.from_host(r, p, s) for r in raws]
+    for groups in (9, 40, 300, 2000):
+        gid = torch.tensor([rng.randrange(groups) for _ in range(rows)], dtype=torch.int32, device="cuda")
+        outs = [torch.zeros(groups * w, dtype=torch.uint8, device="cuda") for w in (133, 133, 8)]
+        arr = (abi.UpColumn * 2)(*[c.up_column() for c in cols])
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        abi.check(lib.up_query_launch(h, arr, 2, rows, gid.data_ptr(), groups, (C.c_void_p * 3)(*[o.data_ptr() for o in outs]),
+                                      err.data_ptr(), torch.cuda.current_stream().cuda_stream), "launch")
+        exp = oracle.query(b, aggs, raws, _raw(gid), rows, groups, threads=8)
+        assert int(err.item()) == 0
+        for k, (o, e) in enumerate(zip(outs, exp)):
+            assert _raw(o) == e, (groups, k)
+    lib.up_module_release(h)

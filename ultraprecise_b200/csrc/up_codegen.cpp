@@ -1548,12 +1548,14 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
             return src.str();
         };
         // fold the cells of ng groups (rep replicas each) into the accumulators
+        // (by threads, not warps: a CTA may be any number of threads)
         src << "template <int S>\nUP_DI void q_cells_flush(const UpQArgs& a, int* cells, int ng, int rep) {\n";
-        src << "    constexpr int WP = " << WP << ";\n    const int lane = threadIdx.x & 31;\n";
-        src << "    if (rep > 1) {\n        for (int it = threadIdx.x >> 5; it < WP * ng; it += blockDim.x >> 5) {\n";
+        src << "    constexpr int WP = " << WP << ";\n";
+        src << "    if (rep > 1) {\n        for (int it = threadIdx.x; it < WP * ng; it += blockDim.x) {\n";
         src << "            const int w = it / ng;\n            int* c = cells + w * S + (it - w * ng) * rep;\n";
-        src << "            int v = 0;\n            if (lane < rep) { v = c[lane]; c[lane] = 0; }\n";
-        src << "            v = __reduce_add_sync(0xffffffffu, v);\n            if (lane == 0) c[0] = v;\n";
+        src << "            int v = 0;\n            for (int k = 0; k < rep; k++) {\n";
+        src << "                int* p = c + ((k + it) & (rep - 1));  // neighbours start in other banks\n";
+        src << "                v += *p;\n                *p = 0;\n            }\n            c[0] = v;\n";
         src << "        }\n        __syncthreads();\n    }\n";
         src << "    for (int it = threadIdx.x; it < ng * " << NR + 1 << "; it += blockDim.x) {\n";
         src << "        const int i = it / ng, g = it - i * ng;\n        int* c = cells + g * rep;\n";
