@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdio>
 #include <map>
+#include <memory>
 #include <set>
 #include <sstream>
 
@@ -276,7 +277,7 @@ struct TEmitter {
     bool out_of_line = false;  // call multiplies and divisions out of line
     bool words = false;        // columns come from a padded shared-memory tile (word loads)
     bool tensor = false;       // wide products on the tensor cores, through a warp's scratch `ws`
-    int scratch_words = 0;     // of a warp, for the products emitted so far
+    int scratch_words = 0, tensor_products = 0;  // a warp's scratch and the number of the products emitted so far
 
     // Operand limbs from which a product goes to the tensor cores: six limbs and
     // the seven bytes of shift fill one 32-byte step of the fragments; the
@@ -284,6 +285,10 @@ struct TEmitter {
     // fixed number of instructions per step.
     static constexpr int kTensorMinLimbs = 6;
     bool on_tensor(int lb) const { return tensor && !out_of_line && K % 4 == 0 && K <= 16 && lb >= kTensorMinLimbs; }
+    void count_tensor(int words) {
+        scratch_words = std::max(scratch_words, words);
+        tensor_products++;
+    }
     static int tc_steps(int lb) { return (4 * lb + 7 + 31) / 32; }
     static int tc_copy(int lb) {
         const int n = (8 * tc_steps(lb) + 4 + 7) / 8;
@@ -344,7 +349,7 @@ struct TEmitter {
         if (on_tensor(np) && f[a].limbs >= np) {
             const std::string c = "TC10_" + std::to_string(d);
             if (tc_p10.insert(d).second) globals << tc_constant(c, p);
-            scratch_words = std::max(scratch_words, tc_words(f[a].limbs, np, true));
+            count_tensor(tc_words(f[a].limbs, np, true));
             body << "    u32 " << t << "[" << K << "]; tpi_mul_const<" << tk() << ", " << f[a].limbs << ", " << np << ">(" << t
                  << ", " << v(a) << ", " << c << ", ws);\n";
             return t;
@@ -399,7 +404,7 @@ struct TEmitter {
                 int a = nd.left, b = nd.right;
                 if (f[a].limbs < f[b].limbs) std::swap(a, b);
                 if (on_tensor(f[b].limbs)) {
-                    scratch_words = std::max(scratch_words, tc_words(f[a].limbs, f[b].limbs, false));
+                    count_tensor(tc_words(f[a].limbs, f[b].limbs, false));
                     body << "    u32 " << v(k) << "[" << K << "]; tpi_mul<" << tk() << ", " << f[a].limbs << ", " << f[b].limbs
                          << ">(" << v(k) << ", " << v(a) << ", " << v(b) << ", ws); u32 " << s(k) << " = " << s(nd.left)
                          << " ^ " << s(nd.right) << ";\n";
@@ -476,6 +481,9 @@ struct TEmitter {
 // 1.14 and 0.73 ms, at p=450 (95 limbs) 0.58 and 0.63 ms, at p=300 (64 limbs, 1M
 // rows) 0.48 and 0.66 ms.
 constexpr int kCoopMinLimbs = 96;
+
+// Shared memory a CTA may have.
+constexpr int kOneCtaSmem = 227 * 1024;
 
 // Widest limb count a cooperative evaluation of the expression needs (every
 // node, every aligned operand, and the headroom of the long divisions), or 0
@@ -725,28 +733,43 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
             if (t > 1) tpiT = t;
         }
         if (tpiT > 0) tpiK = (w + tpiT - 1) / tpiT;
-        // whole groups of four limbs per thread where a product takes the tensor cores
-        if (tpiK >= 3 && tpiK <= 16)
-            for (int k : topo)
-                if (nodes[k].kind == UP_NODE_MUL &&
-                    std::min(f[nodes[k].left].limbs, f[nodes[k].right].limbs) >= TEmitter::kTensorMinLimbs)
-                    tpiK = (tpiK + 3) / 4 * 4;
     }
     out.threads_per_value = tpiT > 0 ? tpiT : 1;
 
     // tile kernel: contiguous columns
     int smem = 0;
     if (tpiT > 0) {
-        TEmitter te(nodes, cols, f, tpiT, tpiK);
-        te.words = true;  // the columns are read from the staged tile below (padded by 16 bytes)
-        te.tensor = true;
-        te.plan(topo);
-        for (int k : topo) te.node(k);
         const int CT = 256;               // CTA threads
         const int G = CT / tpiT;          // values in flight per CTA
+        auto tile_bytes = [&](int rows) {
+            int n = ((rows * BO + 16 + 15) / 16) * 16;
+            for (int c : used) n += ((rows * compact_bytes(cols[c].precision) + 16 + 15) / 16) * 16;
+            return n;
+        };
+        // Products on the tensor cores where some are wide enough, with whole
+        // groups of four limbs per thread (from three on), if their warps'
+        // scratch and a tile of a row per group in flight fit a CTA; else
+        // window products.
+        const int fourK = (tpiK + 3) / 4 * 4;
+        auto emit = [&](bool tensor) {
+            std::unique_ptr<TEmitter> e(new TEmitter(nodes, cols, f, tpiT, tensor ? fourK : tpiK));
+            e->words = true;  // the columns are read from the staged tile below (padded by 16 bytes)
+            e->tensor = tensor;
+            e->plan(topo);
+            for (int k : topo) e->node(k);
+            return e;
+        };
+        auto scratch_bytes = [&](const TEmitter& e) { return CT / 32 * ((e.scratch_words + 3) / 4 * 4) * 4; };
+        std::unique_ptr<TEmitter> tep = emit(tpiK >= 3);
+        const int least = std::max(G, 16);
+        const int smem_cap = kOneCtaSmem;
+        if (tep->tensor && (tep->tensor_products == 0 || tile_bytes(least) + scratch_bytes(*tep) > smem_cap)) tep = emit(false);
+        TEmitter& te = *tep;
+        tpiK = te.K;
         R = 1024;
-        // tensor products run two CTAs per SM, each with room for larger tiles
-        while (R > 16 && (long)R * row_bytes > (te.scratch_words ? 60 : 32) * 1024) R /= 2;
+        // tensor products have room for larger tiles
+        while (R > 16 && (long)R * row_bytes > (te.tensor ? 60 : 32) * 1024) R /= 2;
+        while (te.tensor && R > least && tile_bytes(R) + scratch_bytes(te) > smem_cap) R /= 2;
         std::vector<int> off;
         for (int c : used) {
             off.push_back(smem);
