@@ -5,6 +5,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
+from oracle import oracle
 from ultraprecise_b200 import codec, runtime
 from ultraprecise_b200 import expr as E
 
@@ -44,3 +45,23 @@ def test_products_match_one_thread(p, q, rows):
             m.launch(cols, rows, out=out[:rows * m.value_bytes], err=err)
             assert torch.equal(out[:rows * m.value_bytes], want), (name, tpv)
             assert bool((out[rows * m.value_bytes:] == 0xEE).all()) and int(err.item()) == int(err1.item())
+
+
+# the shorter operand at the limbs from which products go to the tensor cores
+# (6 at 32 threads per value, 16 at 16, 24 at 8, 28 in pairs at 4) and below
+@pytest.mark.parametrize("p,q", [(163, 57), (163, 48), (150, 154), (200, 143), (300, 231), (310, 216), (260, 270), (260, 255),
+                                 (600, 600)])
+def test_products_match_the_oracle(p, q):
+    rows = 333
+    a, b = E.col(0), E.col(1)
+    types = [E.ColType(p, 3), E.ColType(q, 30)]
+    raws = [_column(p, rows, 5), _column(q, rows, 6).view(rows, -1).flip(0).reshape(-1).contiguous()]
+    cols = [runtime.DeviceColumn(t, ty.precision, ty.scale) for t, ty in zip(raws, types)]
+    host = [bytes(t.cpu().numpy().tobytes()) for t in raws]
+    for e in (a * b, a * b + b * a, a * b * E.dec("-7.5") + a):
+        for tpv in (4, 8, 16, 32):
+            m = runtime.compile_expr(e, types, threads_per_value=tpv)
+            err = torch.zeros(1, dtype=torch.int32, device="cuda")
+            out = m.launch(cols, rows, err=err)
+            exp, exp_err = oracle.eval_expr(m.built, m.root, host, rows, m.value_bytes)
+            assert bytes(out.cpu().numpy().tobytes()) == exp and int(err.item()) == exp_err, tpv

@@ -279,12 +279,18 @@ struct TEmitter {
     bool tensor = false;       // wide products on the tensor cores, through a warp's scratch `ws`
     int scratch_words = 0, tensor_products = 0;  // a warp's scratch and the number of the products emitted so far
 
-    // Operand limbs from which a product goes to the tensor cores: six limbs and
-    // the seven bytes of shift fill one 32-byte step of the fragments; the
-    // window product costs a step of shuffles per limb, the tensor one a nearly
-    // fixed number of instructions per step.
-    static constexpr int kTensorMinLimbs = 6;
-    bool on_tensor(int lb) const { return tensor && !out_of_line && K % 4 == 0 && K <= 16 && lb >= kTensorMinLimbs; }
+    // Limbs of the shorter operand from which a product goes to the tensor
+    // cores, by threads per value: the window product costs a step of shuffles
+    // per limb of it, the tensor one a nearly fixed number of instructions per
+    // value, and a warp works through its 32 / T values one after the other.
+    // Measured on B200, window against tensor products in ms: at 32 threads
+    // a*b+c at p=450 with the constant's 12 limbs 0.64 / 0.57; at 16 threads 12
+    // limbs 1.02 / 1.17 (a*b*c at p=110), 16 limbs 1.02 / 0.96, 32 limbs (a*b+c*b at
+    // p=300) 1.07 / 0.62; at 8 threads 21 limbs 0.58 / 0.66, 28 limbs 0.77 / 0.64; at
+    // 4 threads 21 limbs 0.69 / 1.16, 28 limbs 1.49 / 1.11 (a*b+c*b); at 2 threads
+    // 14 limbs 0.48 / 1.68.
+    static int tensor_min_limbs(int t) { return t >= 32 ? 6 : t >= 16 ? 16 : t >= 8 ? 24 : t >= 4 ? 28 : 1 << 30; }
+    bool on_tensor(int lb) const { return tensor && !out_of_line && K % 4 == 0 && K <= 16 && lb >= tensor_min_limbs(T); }
     void count_tensor(int words) {
         scratch_words = std::max(scratch_words, words);
         tensor_products++;
@@ -482,8 +488,9 @@ struct TEmitter {
 // rows) 0.48 and 0.66 ms.
 constexpr int kCoopMinLimbs = 96;
 
-// Shared memory a CTA may have.
-constexpr int kOneCtaSmem = 227 * 1024;
+// Shared memory of a CTA that has an SM to itself, and of one of two (228 KB,
+// 1 KB of each CTA's share reserved).
+constexpr int kOneCtaSmem = 227 * 1024, kTwoCtaSmem = 113 * 1024;
 
 // Widest limb count a cooperative evaluation of the expression needs (every
 // node, every aligned operand, and the headroom of the long divisions), or 0
@@ -747,9 +754,13 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
             return n;
         };
         // Products on the tensor cores where some are wide enough, with whole
-        // groups of four limbs per thread (from three on), if their warps'
-        // scratch and a tile of a row per group in flight fit a CTA; else
-        // window products.
+        // groups of four limbs per thread (from three on), if two CTAs with
+        // their warps' scratch and a tile of a row per group in flight fit an
+        // SM.  One CTA alone hides less of the operands' staging, which only
+        // two or more products make up for: measured on B200 at 8 threads,
+        // window against tensor products, a*b*c at p=380 1.46 / 1.21 ms,
+        // (a+b)*(a-b) at p=600 0.80 / 0.94; a*b*c at p=300 with one CTA 1.19, with
+        // two and half the tile 0.84.
         const int fourK = (tpiK + 3) / 4 * 4;
         auto emit = [&](bool tensor) {
             std::unique_ptr<TEmitter> e(new TEmitter(nodes, cols, f, tpiT, tensor ? fourK : tpiK));
@@ -762,7 +773,9 @@ up_status generate_expr_module(const up_expr_node* nodes, int n_nodes, int root,
         auto scratch_bytes = [&](const TEmitter& e) { return CT / 32 * ((e.scratch_words + 3) / 4 * 4) * 4; };
         std::unique_ptr<TEmitter> tep = emit(tpiK >= 3);
         const int least = std::max(G, 16);
-        const int smem_cap = kOneCtaSmem;
+        const int smem_cap = tile_bytes(least) + scratch_bytes(*tep) <= kTwoCtaSmem ? kTwoCtaSmem
+                             : tep->tensor_products >= 2                           ? kOneCtaSmem
+                                                                                   : 0;
         if (tep->tensor && (tep->tensor_products == 0 || tile_bytes(least) + scratch_bytes(*tep) > smem_cap)) tep = emit(false);
         TEmitter& te = *tep;
         tpiK = te.K;
