@@ -178,6 +178,11 @@ int main(int argc, char** argv) {
     bad += check_mul<16, 8, 8>(n) + check_mul<13, 11, 2>(n) + check_mul<22, 11, 11>(n / 4) + check_mul<32, 16, 16>(n / 8);
     bad += check_mul<64, 32, 32>(n / 32) + check_mul<41, 32, 9>(n / 16);
     bad += check_mul<3, 4, 4>(n) + check_mul<7, 8, 8>(n) + check_mul<20, 16, 16>(n / 8);  // low limbs only
+    // long operands by halves (with small limits when built for that), the
+    // second half as long as the other operand, or a limb shorter
+    bad += check_mul<12, 8, 4>(n) + check_mul<11, 7, 4>(n) + check_mul<13, 8, 5>(n) + check_mul<14, 9, 5>(n);
+    bad += check_mul<16, 12, 4>(n) + check_mul<13, 5, 8>(n) + check_mul<10, 8, 5>(n) + check_mul<9, 9, 5>(n);
+    bad += check_mul<141, 94, 47>(n / 200) + check_mul<187, 125, 63>(n / 200) + check_mul<150, 63, 125>(n / 200);
     bad += check_sums<1, 1, 1>(n) + check_sums<4, 4, 3>(n) + check_sums<5, 5, 5>(n) + check_sums<6, 4, 5>(n);
     bad += check_sums<9, 8, 3>(n) + check_sums<33, 32, 32>(n / 4);
     bad += check_quotient<3, 2>(n) + check_quotient<5, 2>(n) + check_quotient<6, 4>(n) + check_quotient<7, 4>(n);

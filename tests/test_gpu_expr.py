@@ -152,3 +152,18 @@ def test_host_launch_matches_device_launch(p, op, rows, chunk):
     herr = m.launch_host(host, cols, rows, out, chunk_rows=chunk)
     assert bytes(out.numpy().tobytes()) == bytes(want.cpu().numpy().tobytes())
     assert herr == int(err.item())
+
+
+@pytest.mark.parametrize("p", [440, 500])
+def test_wide_products_by_halves(p):
+    """a*b*c with one thread per value: the second product goes by halves of
+    its longer operand; values of all nines and all ones bits among them."""
+    rows = 130
+    rng = random.Random(p)
+    cols = [E.ColType(p, 7)] * 3
+    mod = runtime.compile_expr(E.col(0) * E.col(1) * E.col(2), cols, threads_per_value=1)
+    bits = 8 * codec.compact_bytes(p) - 1
+    special = [0, 1, 10 ** p - 1, (1 << bits) - 1, (1 << bits) - (1 << (bits // 2)), (1 << (bits // 2)) - 1]
+    raws = [codec.encode([(rng.getrandbits(1), rng.choice(special) if rng.random() < 0.5 else rng.randrange(10 ** p))
+                          for _ in range(rows)], p) for _ in range(3)]
+    _check(mod, cols, raws, rows)

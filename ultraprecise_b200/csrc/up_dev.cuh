@@ -235,13 +235,14 @@ UP_DI void add_signed(u32 (&r)[N], u32& sr, const u32 (&a)[NA], u32 sa, const u3
 }
 
 // Half a row of a product: x += a[j] * k at limbs i + j for every second j
-// from J0 (low N limbs).  Neighbouring products fill neighbouring pairs of
-// limbs, so the half row is one chain, its carry ends in the limb above.
-template <int J0, int N, int NA>
+// from J0 up to J1 (low N limbs).  Neighbouring products fill neighbouring
+// pairs of limbs, so the half row is one chain, its carry ends in the limb
+// above; OVER: in the one after that, x being a limb longer there already.
+template <int J0, int J1, bool OVER, int N, int NA>
 UP_DI void mul_row(u32 (&x)[N], const u32 (&a)[NA], u32 k, int i) {
     int top = -1;
 #pragma unroll
-    for (int j = J0; j < NA; j += 2) {
+    for (int j = J0; j < J1; j += 2) {
         const int l = i + j;
         if (l < N) {
             x[l < N ? l : 0] = j == J0 ? mad_lo_cc(a[j], k, x[l < N ? l : 0]) : madc_lo_cc(a[j], k, x[l < N ? l : 0]);
@@ -249,34 +250,66 @@ UP_DI void mul_row(u32 (&x)[N], const u32 (&a)[NA], u32 k, int i) {
         }
         top = l + 2;
     }
-    if (top >= 0 && top < N) x[top >= 0 && top < N ? top : 0] = addc(x[top >= 0 && top < N ? top : 0], 0u);
+    if (top >= 0 && top < N) {
+        if constexpr (OVER) {
+            x[top >= 0 && top < N ? top : 0] = addc_cc(x[top >= 0 && top < N ? top : 0], 0u);
+            if (top + 1 < N) x[top + 1 < N ? top + 1 : 0] = addc(x[top + 1 < N ? top + 1 : 0], 0u);
+        } else {
+            x[top >= 0 && top < N ? top : 0] = addc(x[top >= 0 && top < N ? top : 0], 0u);
+        }
+    }
 }
 
-// r = a * b (low N limbs of the product), a row per limb of b: the even and
-// then the odd products of the row, each a carry chain of one wide
-// multiply-add per product.  Measured on B200 against 64-bit sums per limb:
-// the series at p=100 0.86 -> 0.70 ms, a/b at p=38 0.306 -> 0.282 ms.
-template <int N, int NA, int NB>
+// r += (limbs J0 .. J1-1 of a) * b, a row per limb of b: the even and then the
+// odd products of the row, each a carry chain of one wide multiply-add per
+// product.  Measured on B200 against 64-bit sums per limb: the series at p=100
+// 0.86 -> 0.70 ms, a/b at p=38 0.306 -> 0.282 ms.
+template <int J0, int J1, bool OVER, int N, int NA, int NB>
 UP_DI void mul_rows(u32 (&r)[N], const u32 (&a)[NA], const u32 (&b)[NB]) {
-    zero(r);
 #pragma unroll
     for (int i = 0; i < NB; i++) {
         if (i < N) {
-            mul_row<0>(r, a, b[i], i);
-            mul_row<1>(r, a, b[i], i);
+            mul_row<J0, J1, OVER>(r, a, b[i], i);
+            mul_row<J0 + 1, J1, OVER>(r, a, b[i], i);
         }
+    }
+}
+
+// Products above kMulUnrollPairs whose longer operand is about twice the
+// shorter one go by its halves, up to twice as many pairs: a half, the shorter
+// operand and their product stay in registers, where the whole product and
+// both operands do not (then limbs in local memory, or every row spilled).
+// The first half's product ends at most one limb above the second half's first
+// row, so a row's carry runs on by at most one limb.  Measured on B200, a*b*c
+// with one thread per value: p=450 2.91 -> 1.15 ms (2.18 before carry chains),
+// p=600 4.05 -> 2.28 ms; unrolled without halves p=500 took 3.63 ms, now 1.40.
+UP_DI constexpr bool mul_halves(int na, int nb) {
+    return na * nb > kMulUnrollPairs && na * nb <= 2 * kMulUnrollPairs && na / 2 + 1 >= nb;
+}
+
+// r = a * b (low N limbs), a the longer operand
+template <int N, int NA, int NB>
+UP_DI void mul_long(u32 (&r)[N], const u32 (&a)[NA], const u32 (&b)[NB]) {
+    static_assert(NA >= NB, "a is the longer operand");
+    zero(r);
+    if constexpr (mul_halves(NA, NB)) {
+        constexpr int H = (NA + 1) / 2;
+        mul_rows<0, H, false>(r, a, b);
+        mul_rows<H, NA, (NA - H < NB)>(r, a, b);
+    } else {
+        mul_rows<0, NA, false>(r, a, b);
     }
 }
 
 // r = a * b (low N limbs of the product)
 template <int N, int NA, int NB>
 UP_DI void mul(u32 (&r)[N], const u32 (&a)[NA], const u32 (&b)[NB]) {
-    if constexpr (NA * NB > kPlainPairs && NA * NB <= kMulUnrollPairs) {
-        if constexpr (NA >= NB) mul_rows(r, a, b);
-        else mul_rows(r, b, a);
+    constexpr bool rows = NA * NB <= kMulUnrollPairs || (NA >= NB ? mul_halves(NA, NB) : mul_halves(NB, NA));
+    if constexpr (NA * NB > kPlainPairs && rows) {
+        if constexpr (NA >= NB) mul_long(r, a, b);
+        else mul_long(r, b, a);
     } else {
-        // products above UP_MUL_UNROLL_PAIRS limb pairs keep the outer loop
-        // rolled (compile time)
+        // wider products keep the outer loop rolled (compile time)
         zero(r);
 #pragma unroll((NA * NB <= kPlainPairs) ? NA : 1)
         for (int i = 0; i < NA; i++) {
@@ -308,8 +341,8 @@ UP_DI void mul_u32(u32 (&r)[N], const u32 (&a)[NA], u32 k) {
         }
     } else {
         zero(r);
-        mul_row<0>(r, a, k, 0);
-        mul_row<1>(r, a, k, 0);
+        mul_row<0, NA, false>(r, a, k, 0);
+        mul_row<1, NA, false>(r, a, k, 0);
     }
 }
 
@@ -442,8 +475,8 @@ struct QuotEst {
 // multiply-add per limb.
 template <int NB>
 UP_DI u32 knuth_step(u32 (&w)[NB + 1], const u32 (&nb)[NB], u32 qhat) {
-    mul_row<0>(w, nb, qhat, 0);
-    mul_row<1>(w, nb, qhat, 0);
+    mul_row<0, NB, false>(w, nb, qhat, 0);
+    mul_row<1, NB, false>(w, nb, qhat, 0);
     w[NB] -= qhat;
     if ((int)w[NB] < 0) {
         qhat--;
