@@ -90,3 +90,31 @@ def test_cells_are_folded_by_any_number_of_threads(tmp_path):
     subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-o", exe, cpp], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout
+
+
+def test_cells_fit_the_ctas_they_are_planned_for():
+    """Slots and pieces of the cell kernels, over widths and numbers of sums:
+    the first kernel's within 40 KB, the second's within one of two CTAs of an
+    SM beside the input stages, and never fewer than the first's."""
+    import random
+    rng = random.Random(2)
+    second = 0
+    for _ in range(200):
+        n = rng.randint(1, 10)
+        types = [E.ColType(rng.randint(1, 80), 0) for _ in range(3)]
+        a, b, c = (E.col(i) for i in range(3))
+        exprs = [rng.choice([a * b, a, b - c, a * b * c, a + c]) for _ in range(n)]
+        src = prewarm.query_source(exprs, types, [(abi.UP_AGG_SUM, i) for i in range(n)])
+        inst = [tuple(map(int, m)) for m in re.findall(r"up_query_cells_body<(\d+), (\d+), (\d+), (\d+)>\(a, sm\)", src)]
+        if not inst:
+            continue
+        wp = int(re.search(r"QS = \d+, WP = (\d+)", src).group(1))
+        tags = int(re.search(r"int\* tags = \(int\*\)\(sm \+ (\d+)\);", src).group(1))
+        s, h, _, gmax = inst[0]
+        assert s == h == gmax and (s == 4 or wp * s * 4 <= 40 * 1024)
+        if len(inst) == 2:
+            s2, h2, gmin, gmax2 = inst[1]
+            second += 1
+            assert s2 == gmax2 > s and h2 == 0 and gmin >= s
+            assert tags + wp * s2 * 4 + 32 <= 113 * 1024
+    assert second > 50

@@ -9,7 +9,7 @@ import pytest
 torch = pytest.importorskip("torch")
 
 from oracle import oracle
-from ultraprecise_b200 import abi, codec, runtime
+from ultraprecise_b200 import abi, codec, prewarm, runtime
 from ultraprecise_b200 import expr as E
 
 pytestmark = pytest.mark.gpu
@@ -100,3 +100,33 @@ def test_cells_of_other_cta_sizes(threads):
         for k, (o, e) in enumerate(zip(outs, exp)):
             assert _raw(o) == e, (groups, k)
     lib.up_module_release(h)
+
+
+@pytest.mark.parametrize("p", [9, 18, 38, 140])
+def test_group_counts_at_the_cells_edges(p):
+    """One group less and more than each kernel's cells hold (read from the
+    generated source), by group ids and by two-byte keys whose count stays on
+    the device."""
+    import re
+    exprs, types = [E.col(0) * E.col(1), E.col(0)], [E.ColType(p, 2)] * 2
+    src = prewarm.query_source(exprs, types, AGGS)
+    slots = sorted(int(s) for s in re.findall(r"up_query_cells_body<(\d+), \d+, \d+, \d+>\(a, sm\)", src))
+    assert len(slots) == 2
+    q = runtime.compile_query(exprs, AGGS, types)
+    rng = random.Random(p)
+    for groups in (slots[0], slots[0] + 1, slots[1], slots[1] + 1):
+        rows = groups + 3001
+        cols = [runtime.DeviceColumn(runtime.gen_digits(rows, p, 7 + k), p, 2) for k in range(2)]
+        ids = list(range(groups)) + [int(groups * rng.random() ** 3) for _ in range(rows - groups)]
+        rng.shuffle(ids)
+        gid = torch.tensor(ids, dtype=torch.int32, device="cuda")
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        outs = q.launch(cols, gid, groups, err=err)
+        exp = oracle.query(q.built, q.aggs, [_raw(c.data) for c in cols], _raw(gid), rows, groups, threads=8)
+        keys = [torch.stack([gid // 256, gid % 256], 1).to(torch.uint8).reshape(-1).contiguous()]
+        table = torch.zeros(abi.UP_KEY_TABLE_ENTRIES, dtype=torch.int32, device="cuda")
+        runtime.group_table_from_keys_async(keys, [2], table)
+        got = q.launch_keys_async(cols, keys, [2], table, groups + 5, err=err, rows=rows)
+        assert int(err.item()) == 0
+        for k, e in enumerate(exp):
+            assert _raw(outs[k]) == e and _raw(got[k])[:len(e)] == e, (groups, k)

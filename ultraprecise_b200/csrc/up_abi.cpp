@@ -555,15 +555,19 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
             const bool reg_lo = g.q_gr_lo > 0 && n_groups <= g.q_gr_lo;
             const char* reg_name = keys ? "up_query_tile_rk" : "up_query_tile_r";
             const char* lo_name = keys ? "up_query_tile_rk_lo" : "up_query_tile_r_lo";
-            const char* name = reg_lo                             ? lo_name
-                               : reg                              ? reg_name
-                               : (n_groups <= g.q_gs || a.lacc) ? "up_query_tile_h"
-                                                                  : "up_query_tile_g";
+            const char* name = reg_lo                                               ? lo_name
+                               : reg                                                ? reg_name
+                               : n_groups > g.q_gs_h && n_groups <= g.q_gs ? "up_query_tile_d"
+                               : (n_groups <= g.q_gs || a.lacc)             ? "up_query_tile_h"
+                                                                                    : "up_query_tile_g";
             a.vec_ok = (vec_ok && keys_aligned) ? 1 : 0;
             auto launch_tile = [&](const char* kname) -> cudaError_t {
                 void* k = jit_kernel(*m->jm.ks, kname);
                 const char mode = kname[14];  // up_query_tile_<mode>
-                const int smem = mode == 'h' ? g.q_smem_h : mode == 'r' ? g.q_smem_r : g.q_smem;
+                const int smem = mode == 'h'   ? g.q_smem_h
+                                 : mode == 'd' ? g.q_smem_d
+                                 : mode == 'r' ? g.q_smem_r
+                                               : g.q_smem;
                 const int threads = mode == 'r' ? g.q_threads_r : g.block_threads;
                 const int tile_rows = mode == 'r' ? g.q_tile_rows_r : g.q_tile_rows;
                 const int64_t ntiles = (rows + tile_rows - 1) / tile_rows;
@@ -580,6 +584,7 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
                 if (g.q_gr_lo > 0) e = launch_tile(lo_name);
                 if (e == cudaSuccess && g.q_gr > 0 && n_groups > g.q_gr_lo) e = launch_tile(reg_name);
                 if (e == cudaSuccess && (g.q_gr == 0 || n_groups > g.q_gr)) e = launch_tile("up_query_tile_h");
+                if (e == cudaSuccess && g.q_gs > g.q_gs_h && n_groups > g.q_gs_h) e = launch_tile("up_query_tile_d");
                 if (e == cudaSuccess && n_groups > g.q_gs && !a.lacc) e = launch_tile("up_query_tile_g");
             } else {
                 e = launch_tile(name);

@@ -1211,6 +1211,9 @@ struct NarrowEmitter {
 // Shared memory of a query CTA's cells: with the 32 KB of its two input
 // stages, three CTAs fit on an SM.
 constexpr int kCellBytes = 40 * 1024;
+// Slots of the kernel for more groups than those: within the shared memory of
+// one of two CTAs per SM.
+constexpr int kDirectSlots = 4096;
 
 up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up_col_type* cols, int n_cols,
                                 const up_query_agg* aggs, int n_aggs, const up_compile_opts* opts,
@@ -1437,9 +1440,12 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
     //       table, 3.2 TB/s of column and key bytes;
     //   _h  per-CTA shared-memory cells (cells_add): direct by group id while
     //       the groups fit the S slots (several replicas per group, by lane,
-    //       when they fit that often), else a hash of group ids whose first
-    //       comers keep their slots and whose misses go to limb sums in
-    //       device memory;
+    //       when they fit that often), else, above S2 groups, a hash of group
+    //       ids whose first comers keep their slots and whose misses go to limb
+    //       sums in device memory;
+    //   _d  the same for S < groups <= S2: one cell per group in the shared
+    //       memory of one of two CTAs per SM, where _h keeps four or so for
+    //       fewer groups;
     //   _g  global accumulators: more groups than slots where the limb sums
     //       cannot be used (2^31 rows or more, a caller's scratch too small).
     int row_bytes = 4;
@@ -1467,7 +1473,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
     out.q_staged = staged;
     out.q_tile_rows = R;
     out.q_gr = GR;
-    out.q_gs = 0;
+    out.q_gs = out.q_gs_h = 0;
     out.q_smem = 0;
     if (staged) {
         // one input stage of RT rows: the columns, then group ids or key bytes
@@ -1504,14 +1510,24 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         WP++;
         int S = 2048;
         while (S > 4 && WP * S * 4 > kCellBytes) S /= 2;
+        // More groups than S, up to S2: a kernel with one cell per group and two
+        // CTAs per SM.  S2 is whole warps of slots; where that is no more than S
+        // there is no such kernel.  Measured on B200, 16M rows of SUM(a*b), AVG(a):
+        // at p=38 (S 256, S2 960) 400 groups 1.33 ms hashed, 0.39 ms so; at p=18
+        // (512, 1824) 1000 groups 0.83 and 0.25 ms.  For fewer groups _h is the
+        // faster one: its smaller CTAs are more per SM (p=18, 400 groups 0.17 ms;
+        // with three CTAs of 75 KB 0.20 ms).
+        const int off_tag = 2 * sh.bytes;
+        int S2 = std::min(kDirectSlots, (kTwoCtaSmem - off_tag - 32) / (4 * WP)) / 32 * 32;
+        if (S2 <= S) S2 = S;
         // limb sums of a group: its limbs and its count, in whole 32-byte sectors
         const int NLS = (NLT + 1 + 3) / 4 * 4;
-        const int off_tag = 2 * sh.bytes;
-        const int off_cell = off_tag + S * 4;
-        const int off_hbar = off_cell + (WP * S * 4 + 15) / 16 * 16;
-        out.q_gs = S;
+        auto cells_smem = [&](int slots, int tags) { return off_tag + tags * 4 + (WP * slots * 4 + 15) / 16 * 16 + 16; };
+        out.q_gs_h = S;
+        out.q_gs = S2;
         out.q_limb_words = NLS;
-        out.q_smem_h = off_hbar + 16;
+        out.q_smem_h = cells_smem(S, S);
+        out.q_smem_d = cells_smem(S2, 0);
         int tile_in_bytes = R * 4;
         for (int c : used) tile_in_bytes += R * compact_bytes(cols[c].precision);
         // The tile loop of every staged kernel: the next tile's bulk copies are
@@ -1612,23 +1628,23 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         // queues up on a frequent group's words.  Measured on B200, 8M rows of
         // SUM(a*b), AVG(a), COUNT at p=18 over 100 000 groups of Zipf(1.1)
         // sizes: 12.4 ms with global carry chains, 0.61 ms this way.
-        src << "extern \"C\" __global__ void __launch_bounds__(" << T << ") up_query_tile_h(const UpQArgs a) {\n";
-        src << "    extern __shared__ __align__(128) u8 sm[];\n";
-        src << "    constexpr int R = " << R << ", S = " << S << ", WP = " << WP << ", NLS = " << NLS << ";\n";
-        src << "    u64* bar = (u64*)(sm + " << off_hbar << ");\n";
-        src << "    int* tags = (int*)(sm + " << off_tag << ");\n    int* cells = (int*)(sm + " << off_cell << ");\n";
+        // S: cells, one or more per group for GMIN < groups <= GMAX; H: slots of the
+        // hash for more than QS groups (0: none).
+        src << "template <int S, int H, int GMIN, int GMAX>\nUP_DI void up_query_cells_body(const UpQArgs& a, u8* sm) {\n";
+        src << "    constexpr int R = " << R << ", QS = " << S2 << ", WP = " << WP << ", NLS = " << NLS << ";\n";
+        src << "    int* tags = (int*)(sm + " << off_tag << ");\n    int* cells = tags + H;\n";
+        src << "    u64* bar = (u64*)(sm + " << off_tag << " + H * 4 + (WP * S * 4 + 15) / 16 * 16);\n";
         src << "    const int ng = q_groups(a);\n";
         src << "    if (ng < 0) { if (threadIdx.x == 0 && blockIdx.x == 0 && a.err) atomicOr(a.err, ERR_DOMAIN); return; }\n";
-        src << "    if (ng <= " << GR << ") return;  // the register kernels'\n";
-        src << "    const bool hashed = ng > S;\n    if (hashed && !a.lacc) return;\n";
+        src << "    const bool hashed = H > 0 && ng > QS;\n    if (hashed ? !a.lacc : ng <= GMIN || ng > GMAX) return;\n";
         src << "    int rep = 1;  // replicas per group: lanes of a warp rarely meet on a cell\n";
         src << "    if (!hashed)\n        for (rep = 32; ng * rep > S;) rep >>= 1;\n";
         src << "    const int lane = threadIdx.x & 31;\n";
         src << "    for (int i = threadIdx.x; i < WP * S; i += blockDim.x) cells[i] = 0;\n";
-        src << "    for (int i = threadIdx.x; i < S; i += blockDim.x) tags[i] = -1;\n";
+        src << "    for (int i = threadIdx.x; i < H; i += blockDim.x) tags[i] = -1;\n";
         src << "    // fold the cells into the accumulators (every thread of the CTA)\n";
         src << "    auto flush = [&]() {\n        if (hashed) {\n";
-        src << "            for (int s = threadIdx.x; s < S; s += blockDim.x) {\n";
+        src << "            for (int s = threadIdx.x; s < H; s += blockDim.x) {\n";
         src << "                int* c = cells + s;\n                const int n = c[(WP - 1) * S];\n";
         src << "                if (n == 0) continue;\n                i64* l = a.lacc + (i64)tags[s] * NLS;\n                i64 v;\n";
         for (int i = 0; i < NR; i++)
@@ -1651,7 +1667,8 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
                 src << "in + " << off[i] << " + r * " << compact_bytes(cols[used[i]].precision) << ", ";
             src << "3" << margs() << ");\n";
         }
-        src << "            const int s = hashed ? cell_slot<S>(tags, g) : g * rep + (lane & (rep - 1));\n";
+        src << "            int s;\n            if constexpr (H > 0) s = hashed ? cell_slot<H>(tags, g) : g * rep + (lane & (rep - 1));\n";
+        src << "            else s = g * rep + (lane & (rep - 1));\n";
         src << "            if (s >= 0) {\n                int* c = cells + s;\n";
         for (int i = 0; i < NR; i++)
             src << "                cells_add<S, " << np[i] << ">(c + " << cell_off[i] << " * S, qm" << i << ", qs" << i << ");\n";
@@ -1666,13 +1683,20 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         src << "    err = __reduce_or_sync(0xffffffffu, err);\n";
         src << "    if ((threadIdx.x & 31) == 0 && err != 0u && a.err) atomicOr(a.err, err);\n";
         src << "}\n\n";
+        auto cells_kernel = [&](const char* name, int slots, int tags, int gmin) {
+            src << "extern \"C\" __global__ void __launch_bounds__(" << T << ") " << name
+                << "(const UpQArgs a) {\n    extern __shared__ __align__(128) u8 sm[];\n    up_query_cells_body<" << slots << ", " << tags
+                << ", " << gmin << ", " << slots << ">(a, sm);\n}\n\n";
+        };
+        cells_kernel("up_query_tile_h", S, S, GR);
+        if (S2 > S) cells_kernel("up_query_tile_d", S2, 0, std::max(GR, S));
         // _g: carry chains of global atomics (see the modes above)
         src << "extern \"C\" __global__ void __launch_bounds__(" << T << ") up_query_tile_g(const UpQArgs a) {\n";
         src << "    extern __shared__ __align__(128) u8 sm[];\n";
         src << "    constexpr int R = " << R << ";\n    u64* bar = (u64*)(sm + " << 2 * sh.bytes << ");\n";
         src << "    const int ng = q_groups(a);\n";
         src << "    if (ng < 0) { if (threadIdx.x == 0 && blockIdx.x == 0 && a.err) atomicOr(a.err, ERR_DOMAIN); return; }\n";
-        src << "    if (ng <= " << S << " || a.lacc) return;\n";
+        src << "    if (ng <= " << S2 << " || a.lacc) return;\n";
         src << "    const i64 ntiles = (a.rows + R - 1) / R;\n";
         src << "    const i64 nfull = a.vec_ok ? a.rows / R : 0;  // tiles moved by bulk copies\n";
         src << "    u32 err = 0u;\n" << tile_pipeline_open(sh);
@@ -1887,6 +1911,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
             out.kernels.push_back("up_query_tile_rk_lo");
         }
         out.kernels.push_back("up_query_tile_h");
+        if (out.q_gs > out.q_gs_h) out.kernels.push_back("up_query_tile_d");
         out.kernels.push_back("up_query_tile_g");
     }
     out.block_threads = T;

@@ -98,10 +98,12 @@ struct GeneratedModule {
     int q_tile_rows = 0;          // rows per tile of the tile kernels
     int q_gr = 0;                 // up_query_tile_r handles n_groups <= q_gr
     int q_gr_lo = 0;              // up_query_tile_r_lo handles n_groups <= q_gr_lo (0: no such kernel)
-    int q_gs = 0;                 // slots of up_query_tile_h's cells: direct for n_groups <= q_gs, else hashed
+    int q_gs = 0;                 // groups with a cell each: direct for n_groups <= q_gs, else hashed
+    int q_gs_h = 0;               // of them up_query_tile_h's (which also hashes); up_query_tile_d takes the rest
     int q_limb_words = 0;         // 64-bit words of one group's limb sums (hashed launches)
     int q_smem = 0;               // dynamic shared memory of up_query_tile_g
     int q_smem_h = 0;             // of up_query_tile_h
+    int q_smem_d = 0;             // of up_query_tile_d
     // the register kernels' shared memory, threads and rows per tile
     int q_smem_r = 0, q_threads_r = 0, q_tile_rows_r = 0;
     long work_per_row = 0;        // limb-product work + bytes per row (scheduling cost estimate)
