@@ -106,3 +106,31 @@ def test_columns_met_in_any_order(groups):
         assert int(err.item()) == 0
         for k, (o, e) in enumerate(zip(outs, exp)):
             assert _raw(o) == e, f"aggregate {k}"
+
+
+@pytest.mark.parametrize("p,word", [(9, torch.int32), (18, torch.int64)])
+def test_register_sums_are_folded_several_times(p, word):
+    """Two folds and more of the register sums in every CTA (each takes 256
+    tiles of 1024 rows between them): sums of two words (products) and of three
+    (values of 61 bits), of both signs, against the sums of one period."""
+    period, times = 42, 16_000_000
+    top = 10 ** p // 40 if word is torch.int32 else (1 << 59) - 1
+    vals = [(-1) ** (i % 5) * (top - 7 * i) for i in range(period)]
+    sign = 1 << (8 * codec.compact_bytes(p) - 1)
+    raw = [v if v >= 0 else (-v | sign) - 2 * sign for v in vals]
+    a = torch.tensor(raw, dtype=word, device="cuda").repeat(times)
+    keys = [torch.tensor([i % 3 + 65 for i in range(period)], dtype=torch.uint8, device="cuda").repeat(times)]
+    x = E.col(0)
+    exprs = [x * E.lit(-31)] if word is torch.int32 else [x, -x + E.lit(1)]
+    factor = [lambda v: -31 * v] if word is torch.int32 else [lambda v: v, lambda v: 1 - v]
+    aggs = [(abi.UP_AGG_SUM, i) for i in range(len(exprs))] + [(abi.UP_AGG_COUNT, 0)]
+    q = runtime.compile_query(exprs, aggs, [E.ColType(p, 0)])
+    table = torch.zeros(abi.UP_KEY_TABLE_ENTRIES, dtype=torch.int32, device="cuda")
+    runtime.group_table_from_keys_async(keys, [1], table)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = q.launch_keys_async([runtime.DeviceColumn(a.view(torch.uint8), p, 0)], keys, [1], table, 4, err=err, rows=period * times)
+    assert int(err.item()) == 0
+    for k, f in enumerate(factor):
+        got = [-d["mag"] if d["sign"] else d["mag"] for d in codec.decode_agg(_raw(outs[k])[:3 * abi.UP_AGG_DECIMAL_BYTES], 3)]
+        assert got == [times * sum(f(v) for i, v in enumerate(vals) if i % 3 == g) for g in range(3)], k
+    assert outs[-1].view(torch.int64)[:3].tolist() == [14 * times] * 3

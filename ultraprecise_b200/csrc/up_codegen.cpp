@@ -1208,6 +1208,9 @@ struct NarrowEmitter {
     }
 };
 
+// Tiles of a query CTA between two folds of its register sums.
+constexpr int kFoldTiles = 256;
+
 // Shared memory of a query CTA's cells: with the 32 KB of its two input
 // stages, three CTAs fit on an SM.
 constexpr int kCellBytes = 40 * 1024;
@@ -1821,9 +1824,10 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
             for (int i = 0; i < NR; i++)
                 src << "                cells_add<S, " << np[i] << ">(c + " << cell_off[i] << " * S, qm" << i << ", qs" << i << ");\n";
             src << "            }\n        }\n        __syncthreads();\n";
-            // cells stay exact for kCellRows rows, register sums for 2^15 per thread
+            // cells stay exact for kCellRows rows, register sums for 2^15 per
+            // thread: folded at a 32nd of that, for next to nothing
             src << "        if ((k + 1) % (kCellRows / R) == 0 && __syncthreads_or(wide)) { q_cells_flush<S>(a, cells, ng, 32); wide = false; }\n";
-            src << "        if ((k + 1) % 8192 == 0) flush_regs();\n    }\n";
+            src << "        if ((k + 1) % " << kFoldTiles << " == 0) flush_regs();\n    }\n";
             src << "    if (__syncthreads_or(wide)) q_cells_flush<S>(a, cells, ng, 32);\n    flush_regs();\n" << tile_pipeline_close();
             src << "    if (KEYS && matched != nrow) err |= ERR_DOMAIN;  // a key outside the table\n";
             src << "    err = __reduce_or_sync(0xffffffffu, err);\n";
