@@ -134,3 +134,37 @@ def test_register_sums_are_folded_several_times(p, word):
         got = [-d["mag"] if d["sign"] else d["mag"] for d in codec.decode_agg(_raw(outs[k])[:3 * abi.UP_AGG_DECIMAL_BYTES], 3)]
         assert got == [times * sum(f(v) for i, v in enumerate(vals) if i % 3 == g) for g in range(3)], k
     assert outs[-1].view(torch.int64)[:3].tolist() == [14 * times] * 3
+
+
+@pytest.mark.parametrize("groups,keys", [(3, False), (7, False), (6, True)])
+def test_runs_of_wide_and_narrow_tiles(groups, keys):
+    """Tiles of wide rows, of narrow ones and of both in turn, several per CTA:
+    after tiles of wide rows the kernels evaluate whole tiles the general way."""
+    import numpy as np
+    rng = np.random.default_rng(groups)
+    rows, p = 2_400_000, 18
+    tiles = rows // 1024 + 1
+    kind = rng.integers(0, 3, tiles // 37 + 1).repeat(37)[:tiles].repeat(1024)[:rows]  # 0 narrow, 1 wide, 2 mixed
+    wide = (kind == 1) | ((kind == 2) & (rng.random(rows) < 0.3))
+    raws = []
+    for _ in range(2):
+        v = np.where(wide, rng.integers(0, 10 ** 18, rows), rng.integers(0, 1_000_000, rows)) * rng.choice([-1, 1], rows)
+        raws.append(codec.np_compact_from_int64(v, p).tobytes())
+    a, b = E.col(0), E.col(1)
+    exprs = [a * b, b - a]
+    aggs = [(abi.UP_AGG_SUM, 0), (abi.UP_AGG_AVG, 1), (abi.UP_AGG_COUNT, 0)]
+    q = runtime.compile_query(exprs, aggs, [E.ColType(p, 2)] * 2)
+    cols = [runtime.DeviceColumn.from_host(r, p, 2) for r in raws]
+    gid = torch.from_numpy(rng.integers(0, groups, rows).astype(np.int32)).cuda()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    if keys:
+        key = [gid.to(torch.uint8)]
+        table = torch.zeros(abi.UP_KEY_TABLE_ENTRIES, dtype=torch.int32, device="cuda")
+        runtime.group_table_from_keys_async(key, [1], table)
+        outs = q.launch_keys_async(cols, key, [1], table, 8, err=err, rows=rows)
+    else:
+        outs = q.launch(cols, gid, groups, err=err)
+    exp = oracle.query(q.built, q.aggs, raws, _raw(gid), rows, groups, threads=8)
+    assert int(err.item()) == 0
+    for k, (o, e) in enumerate(zip(outs, exp)):
+        assert _raw(o)[:len(e)] == e, f"aggregate {k}"
