@@ -39,7 +39,7 @@ def test_indexed_rows_equal_contiguous_rows(p, shift, out_shift, rows):
     assert bool((buf[:out_shift] == 0xEE).all()) and bool((buf[out_shift + n * m.value_bytes:] == 0xEE).all())
 
 
-@pytest.mark.parametrize("p", [3, 9, 16, 18, 38, 77])
+@pytest.mark.parametrize("p", [3, 9, 12, 15, 16, 18, 38, 77])
 @pytest.mark.parametrize("rows", [1, 255, 1025])
 def test_nullable_rows(p, rows):
     s = min(2, p - 1)
