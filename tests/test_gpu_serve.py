@@ -150,3 +150,37 @@ def test_session_merges_same_module_requests(shapes):
     assert st["completed"] == 60 and st["failed"] == 0
     assert st["merged_launches"] >= 1 and st["merged_requests"] >= 2
     sess.close()
+
+
+def test_grouped_request_at_the_accumulators_size():
+    """A query with more groups than cells whose outputs and accumulators just
+    fit the session's budget is admitted, though its limb sums would not fit."""
+    rows, groups, p = 40_000, 12_000, 18
+    aggs = [(abi.UP_AGG_SUM, 0), (abi.UP_AGG_AVG, 1), (abi.UP_AGG_COUNT, 0)]
+    q = runtime.compile_query([E.col(0) * E.col(1), E.col(0)], aggs, [E.ColType(p, 2)] * 2)
+    cols = [runtime.DeviceColumn(runtime.gen_digits(rows, p, 3 + k), p, 2) for k in range(2)]
+    gid = torch.randint(0, groups, (rows,), dtype=torch.int32, device="cuda",
+                        generator=torch.Generator(device="cuda").manual_seed(1))
+    alone = [bytes(o.cpu().numpy().tobytes()) for o in q.launch(cols, gid, groups)]
+
+    def pad(n):
+        return (n + 255) // 256 * 256
+
+    words = 6 + 4  # accumulators of 126 and of 63 bits, a sign and 40 bits of rows
+    cap = 256 + 2 * pad(groups * 133) + pad(groups * 8) + pad(groups * words * 4 + 16) + pad(groups * 8)
+    sess = serve.Session(n_streams=2, memory_cap_bytes=cap)
+    for _ in range(2):
+        rid = sess.submit(q, cols, rows, gid, groups)
+        assert sess.wait(rid, 60_000) == serve.DONE
+        for part in range(3):
+            out, err = sess.result(rid, part)
+            assert err == 0 and bytes(out.cpu().numpy().tobytes()) == alone[part]
+        sess.release(rid)
+    assert sess.stats()["max_outstanding_bytes"] <= cap
+    with pytest.raises(abi.UpError):
+        serve_small = serve.Session(n_streams=2, memory_cap_bytes=cap - 4096)
+        try:
+            serve_small.submit(q, cols, rows, gid, groups)
+        finally:
+            serve_small.close()
+    sess.close()

@@ -487,7 +487,7 @@ size_t query_scratch_bytes_max(const GeneratedModule& g, int32_t n_groups) {
 
 up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64_t rows, const int32_t* group_ids,
                           int32_t n_groups, void* const* outs, uint32_t* err_word, void* stream, bool spread,
-                          const QueryKeys* keys, void* caller_scratch, size_t caller_scratch_bytes) {
+                          const QueryKeys* keys, void* caller_scratch, size_t scratch_bytes) {
     if (!m || !m->is_query) return fail(UP_ERR_INVALID_ARG, "not a query module");
     const bool device_count = keys && keys->capacity > 0;
     if (device_count) n_groups = keys->capacity;  // accumulators and outputs sized for the capacity
@@ -508,26 +508,40 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
     if (sm_count_current() <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t accw = (size_t)std::max(g.acc_words_per_group, 1);
-    size_t need = query_scratch_bytes(g, n_groups);
     // More groups than cells: limb sums, which stay exact below 2^31 rows
     // (every sum adds signed 32-bit limbs in 64 bits).  A count known on the
     // host needs no accumulators beside them; a count on the device may turn
-    // out small enough for the cells, whose accumulators it keeps.
+    // out small enough for the cells, whose accumulators it keeps.  Where they
+    // do not fit the caller's scratch or limit, or the device, the accumulators
+    // alone do, as for 2^31 rows.
     bool limbs = contig && g.q_staged && g.q_gs > 0 && n_groups > g.q_gs && rows < ((int64_t)1 << 31);
-    const int32_t acc_groups = limbs ? (device_count ? g.q_gs : 0) : n_groups;
-    const size_t limb_off = (query_scratch_bytes(g, acc_groups) + 31u) & ~(size_t)31u;
-    const size_t limb_need = limb_off + (size_t)n_groups * g.q_limb_words * 8u;
-    if (limbs && caller_scratch && limb_need > caller_scratch_bytes) limbs = false;
-    if (limbs) need = limb_need;
-    const size_t acc_bytes = (((size_t)(limbs ? acc_groups : n_groups) * accw * 4u) + 15u) & ~(size_t)15u;
+    size_t acc_bytes = 0, limb_off = 0, need = 0;
+    auto size_scratch = [&]() {
+        const int32_t acc_groups = limbs ? (device_count ? g.q_gs : 0) : n_groups;
+        acc_bytes = (((size_t)acc_groups * accw * 4u) + 15u) & ~(size_t)15u;
+        limb_off = (query_scratch_bytes(g, acc_groups) + 31u) & ~(size_t)31u;
+        need = limbs ? limb_off + (size_t)n_groups * g.q_limb_words * 8u : query_scratch_bytes(g, n_groups);
+    };
+    size_scratch();
+    if (limbs && scratch_bytes > 0 && need > scratch_bytes) {
+        limbs = false;
+        size_scratch();
+    }
     void* scratch = caller_scratch;
     if (caller_scratch) {
-        if (need > caller_scratch_bytes)
+        if (need > scratch_bytes)
             return fail(UP_ERR_INVALID_ARG, "scratch too small: " + std::to_string(n_groups) + " groups need " +
-                                                std::to_string(need) + " bytes, " +
-                                                std::to_string(caller_scratch_bytes) + " given");
+                                                std::to_string(need) + " bytes, " + std::to_string(scratch_bytes) +
+                                                " given");
     } else {
-        UP_CUDA(scratch_alloc(&scratch, need, s));
+        cudaError_t ea = scratch_alloc(&scratch, need, s);
+        if (ea == cudaErrorMemoryAllocation && limbs) {
+            cudaGetLastError();
+            limbs = false;
+            size_scratch();
+            ea = scratch_alloc(&scratch, need, s);
+        }
+        if (ea != cudaSuccess) return cuda_fail(ea, "scratch allocation");
     }
     cudaError_t e = cudaMemsetAsync(scratch, 0, need, s);
     a.rows = rows;

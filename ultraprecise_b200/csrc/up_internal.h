@@ -252,7 +252,9 @@ size_t query_scratch_bytes(const upi::GeneratedModule& g, int32_t n_groups);
 size_t query_scratch_bytes_max(const upi::GeneratedModule& g, int32_t n_groups);
 // scratch: caller-provided device memory of scratch_bytes (at least
 // query_scratch_bytes, 16-byte aligned) used instead of a stream-ordered
-// allocation; the launch clears what it uses on `stream`.
+// allocation; the launch clears what it uses on `stream`.  Without it,
+// scratch_bytes > 0 is the most the launch may allocate (query_scratch_bytes or
+// more).
 up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64_t rows, const int32_t* group_ids,
                           int32_t n_groups, void* const* outs, uint32_t* err_word, void* stream, bool spread,
                           const QueryKeys* keys = nullptr, void* scratch = nullptr, size_t scratch_bytes = 0);

@@ -33,6 +33,7 @@ struct Req {
     double done_ms = 0.0;
     int32_t state = UP_REQ_QUEUED;
     int64_t bytes = 0;                  // outputs + query scratch, for admission
+    size_t scratch_limit = 0;           // > 0: the most scratch the query may allocate
     std::vector<int64_t> part_off, part_bytes;
     int64_t out_bytes = 0;              // the allocation: err word slot + outputs
     bool heavy = false;                 // work above opts.heavy_work: low-priority stream, spread grid
@@ -94,7 +95,9 @@ void CUDART_CB on_done(void* p) {
 
 // Bytes a request needs while it runs: its outputs (plus the err slot) and,
 // for queries, the accumulator scratch up_query_launch allocates.
-void size_request(Req& r, double heavy_work) {
+// A query whose faster limb sums alone would not fit the session's budget is
+// launched within its accumulators.
+void size_request(Req& r, double heavy_work, int64_t budget) {
     const GeneratedModule& g = r.module->jm.gen;
     r.part_off.clear();
     r.part_bytes.clear();
@@ -112,6 +115,10 @@ void size_request(Req& r, double heavy_work) {
             off += pad((int64_t)r.n_groups * w);
         }
         r.bytes = off + pad((int64_t)query_scratch_bytes_max(g, r.n_groups) + 16);
+        if (r.bytes > budget) {
+            r.scratch_limit = query_scratch_bytes(g, r.n_groups);
+            r.bytes = off + pad((int64_t)r.scratch_limit + 16);
+        }
     }
     r.out_bytes = off;
     r.heavy = heavy_work > 0 && (double)r.rows * (double)g.work_per_row > heavy_work;
@@ -137,7 +144,7 @@ void launch(up_serve* s, Req* r) {
             std::vector<void*> outs;
             for (size_t k = 0; k < r->part_off.size(); k++) outs.push_back((uint8_t*)r->mem + r->part_off[k]);
             status = query_launch_ex(r->module, r->in.data(), (int32_t)r->in.size(), r->rows, r->group_ids,
-                                     r->n_groups, outs.data(), err, st, r->heavy);
+                                     r->n_groups, outs.data(), err, st, r->heavy, nullptr, nullptr, r->scratch_limit);
         }
     }
     if (status == UP_OK) {
@@ -350,8 +357,8 @@ up_status up_serve_submit(up_serve* s, const up_serve_request* req, int64_t* id)
     r->group_ids = req->group_ids;
     r->n_groups = req->n_groups;
     r->owner = s;
-    size_request(*r, s->opts.heavy_work);
     std::lock_guard<std::mutex> g(s->mu);
+    size_request(*r, s->opts.heavy_work, s->budget);
     if (r->bytes > s->budget) return fail(UP_ERR_NO_MEMORY, "request larger than the session's memory budget");
     r->arrival_ms = req->arrival_ms >= 0 ? req->arrival_ms : s->now_ms();
     r->id = s->next_id++;
