@@ -3,6 +3,7 @@
 
 #include <atomic>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -102,7 +103,7 @@ int resident_ctas(void* kernel, int threads, int smem) {
     return n;
 }
 
-// Shared memory above 48 KB is asked for once per kernel and device, together
+// Shared memory above 48 KB is asked for once per kernel and context, together
 // with the CTAs per SM; 0: refused.
 template <int (*Find)(void*, int, int)>
 int prepared(void* kernel, int threads, int smem) {
@@ -114,17 +115,11 @@ int prepared(void* kernel, int threads, int smem) {
     return Find(kernel, threads, smem);
 }
 
-// CTAs of a looping launch: the resident ones of every SM of the current
-// device; <= 0 when there is no device or the kernel cannot run on it.
+// CTAs of a looping launch: the resident ones of each of `sms` SMs; <= 0 when
+// the kernel cannot run there.
 template <int (*Find)(void*, int, int)>
-int64_t resident_grid(const up_module* m, void* kernel, int threads, int smem) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    const int sms = sm_count_current();
-    return sms <= 0 ? 0 : (int64_t)sms * jit_resident(*m->jm.ks, kernel, dev, threads, smem, prepared<Find>);
+int64_t resident_grid(const up_module* m, void* kernel, int threads, int smem, int sms) {
+    return (int64_t)sms * jit_resident(*m->jm.ks, kernel, context_id(), threads, smem, prepared<Find>);
 }
 
 }  // namespace
@@ -146,9 +141,33 @@ int sm_count_current() {
     return n;
 }
 
+// The current context's id: unique over the process's life, so that a device
+// that was reset is told from the one before.  0 where there is no context yet
+// (a thread's first call) or no way to ask.
+uint64_t context_id() {
+    using Fn = int (*)(void* context, unsigned long long* id);  // cuCtxGetId
+    static const Fn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (Fn)f;
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == 0 ? id : 0;
+}
+
+namespace {
+// The scratch pools by context; one whose context is gone went with it and is
+// not touched again.
+std::mutex g_pools_mu;
+std::map<uint64_t, cudaMemPool_t> g_pools;
+}  // namespace
+
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64];  // by device, kept to the process's end
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -160,24 +179,30 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
         capturing = cudaStreamCaptureStatusActive;
     }
     cudaMemPool_t pool = nullptr;
-    if (dev < 64 && capturing == cudaStreamCaptureStatusNone) {
-        std::lock_guard<std::mutex> g(mu);
-        if (!pools[dev]) {
+    const uint64_t ctx = capturing == cudaStreamCaptureStatusNone ? context_id() : 0;
+    if (ctx != 0) {
+        std::lock_guard<std::mutex> g(g_pools_mu);
+        auto it = g_pools.find(ctx);
+        if (it == g_pools.end()) {
             cudaMemPoolProps props = {};
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
             uint64_t keep = kScratchKeep;
             cudaMemPool_t made = nullptr;
-            if (cudaMemPoolCreate(&made, &props) == cudaSuccess &&
-                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
-                pools[dev] = made;
-            } else {
+            // another thread's capture must not end because of this
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (cudaMemPoolCreate(&made, &props) != cudaSuccess ||
+                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
                 cudaGetLastError();
                 if (made) cudaMemPoolDestroy(made);
+                made = nullptr;
             }
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (made) it = g_pools.emplace(ctx, made).first;
         }
-        pool = pools[dev];
+        if (it != g_pools.end()) pool = it->second;
     }
     return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
 }
@@ -264,10 +289,11 @@ up_status up_expr_launch_many(up_module* m, const up_column* in, int32_t n_in, c
         if (st != UP_OK) return st;
     }
     if (reqs.empty()) return UP_OK;
-    if (sm_count_current() <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
+    const int sms = sm_count_current();
+    if (sms <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
     void* k = jit_kernel(*m->jm.ks, "up_expr_multi");
     if (!k) return fail(UP_ERR_CUDA, "module has no up_expr_multi kernel");
-    const int64_t cap = resident_grid<occupancy>(m, k, g.multi_threads, g.multi_smem);
+    const int64_t cap = resident_grid<occupancy>(m, k, g.multi_threads, g.multi_smem, sms);
     if (cap <= 0) return fail(UP_ERR_CUDA, "shared memory of up_expr_multi refused");
     UpMultiReq* d = nullptr;
     const size_t bytes = reqs.size() * sizeof(UpMultiReq);
@@ -338,13 +364,14 @@ up_status expr_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64_
     a.out_nullable = g.out_bytes != (g.out_is_compare ? 1 : compact_bytes(g.out_precision));
     vec_ok = vec_ok && aligned16(out);
     a.vec_ok = vec_ok ? 1 : 0;
-    if (sm_count_current() <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
+    const int sms = sm_count_current();
+    if (sms <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
     void* args[1] = {&a};
     cudaStream_t s = (cudaStream_t)stream;
     if (contig && !a.out_nullable) {
         void* k = jit_kernel(*m->jm.ks, "up_expr_tile");
         const int64_t ntiles = (rows + g.tile_rows - 1) / g.tile_rows;
-        const int64_t resident = resident_grid<resident_ctas>(m, k, g.block_threads, g.smem_bytes);
+        const int64_t resident = resident_grid<resident_ctas>(m, k, g.block_threads, g.smem_bytes, sms);
         if (resident <= 0) return fail(UP_ERR_CUDA, "shared memory of up_expr_tile refused");
         const int64_t cap = spread ? (int64_t)INT32_MAX : resident;
         const unsigned grid = (unsigned)std::min<int64_t>(ntiles, cap);
@@ -353,7 +380,7 @@ up_status expr_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64_
         void* k = jit_kernel(*m->jm.ks, "up_expr_generic");
         const int64_t blocks = (rows + g.block_threads - 1) / g.block_threads;
         const int64_t cap =
-            spread ? (int64_t)INT32_MAX : resident_grid<occupancy>(m, k, g.block_threads, 0) * 4;
+            spread ? (int64_t)INT32_MAX : resident_grid<occupancy>(m, k, g.block_threads, 0, sms) * 4;
         const unsigned grid = (unsigned)std::min<int64_t>(blocks, cap);
         UP_CUDA(cudaLaunchKernel((const void*)k, dim3(grid), dim3(g.block_threads), args, 0, s));
     }
@@ -505,7 +532,8 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
         if (!outs[k]) return fail(UP_ERR_INVALID_ARG, "output " + std::to_string(k) + " is NULL");
         a.out[k] = (uint8_t*)outs[k];
     }
-    if (sm_count_current() <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
+    const int sms = sm_count_current();
+    if (sms <= 0) return fail(UP_ERR_NO_DEVICE, "no CUDA device");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t accw = (size_t)std::max(g.acc_words_per_group, 1);
     // More groups than cells: limb sums, which stay exact below 2^31 rows
@@ -587,7 +615,7 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
                 const int64_t ntiles = (rows + tile_rows - 1) / tile_rows;
                 // the register and shared-memory modes merge once per CTA, so a
                 // spread launch keeps a bounded grid of several waves
-                const int64_t cap = resident_grid<occupancy>(m, k, threads, smem) * (spread ? 8 : 1);
+                const int64_t cap = resident_grid<occupancy>(m, k, threads, smem, sms) * (spread ? 8 : 1);
                 if (cap <= 0) return cudaErrorInvalidValue;
                 return cudaLaunchKernel((const void*)k, dim3((unsigned)std::min<int64_t>(ntiles, cap)),
                                         dim3(threads), args, (size_t)smem, s);
@@ -606,7 +634,7 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
         } else {
             void* k = jit_kernel(*m->jm.ks, "up_query_acc");
             const int64_t blocks = (rows + g.block_threads - 1) / g.block_threads;
-            const int64_t cap = resident_grid<occupancy>(m, k, g.block_threads, 0) * 4;
+            const int64_t cap = resident_grid<occupancy>(m, k, g.block_threads, 0, sms) * 4;
             e = cudaLaunchKernel((const void*)k, dim3((unsigned)std::min<int64_t>(blocks, cap)), dim3(g.block_threads),
                                  args, 0, s);
         }

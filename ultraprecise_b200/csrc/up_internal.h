@@ -159,15 +159,17 @@ up_status jit_load(const std::vector<char>& cubin, const std::vector<std::string
 up_status jit_get(const GeneratedModule& gen, std::shared_ptr<JitKernelSet>& out);
 void* jit_kernel(const JitKernelSet& ks, const std::string& name);  // cudaKernel_t as void*
 int jit_cache_size(bool clear);
-// CTAs per SM a kernel of the set is launched with on `device`: what `find`
-// returned for it the first time (<= 0, a failure, is not kept).
-int jit_resident(const JitKernelSet& ks, void* kernel, int device, int threads, int smem,
+// CTAs per SM a kernel of the set is launched with in `context` (context_id):
+// what `find` returned for it the first time (<= 0, a failure, is not kept, nor
+// anything for context 0).
+int jit_resident(const JitKernelSet& ks, void* kernel, uint64_t context, int threads, int smem,
                  int (*find)(void* kernel, int threads, int smem));
 const std::string& device_header_source();
 
 // ------------------------------------------------------------ devices
 int sm_count_current();
-// Stream-ordered scratch from the library's own pool of the current device,
+uint64_t context_id();
+// Stream-ordered scratch from the library's own pool of the current context,
 // freed by cudaFreeAsync.  The pool keeps up to kScratchKeep bytes over a
 // synchronisation, where the default pool gives everything back to the driver
 // and the next launch allocates anew (0.4 ms and more on B200).

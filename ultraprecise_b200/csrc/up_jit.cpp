@@ -50,10 +50,10 @@ struct JitKernelSet {
     std::vector<char> cubin;
     cudaLibrary_t lib = nullptr;
     std::map<std::string, cudaKernel_t> kernels;
-    // resident CTAs per SM of a kernel's launches, by device, threads and
+    // resident CTAs per SM of a kernel's launches, by context, threads and
     // shared memory (found out at the first launch of each)
     mutable std::mutex mu;
-    mutable std::map<std::tuple<void*, int, int, int>, int> resident;
+    mutable std::map<std::tuple<void*, uint64_t, int, int>, int> resident;
     ~JitKernelSet() {
         if (lib) cudaLibraryUnload(lib);
     }
@@ -490,9 +490,10 @@ void* jit_kernel(const JitKernelSet& ks, const std::string& name) {
     return it == ks.kernels.end() ? nullptr : (void*)it->second;
 }
 
-int jit_resident(const JitKernelSet& ks, void* kernel, int device, int threads, int smem,
+int jit_resident(const JitKernelSet& ks, void* kernel, uint64_t context, int threads, int smem,
                  int (*find)(void* kernel, int threads, int smem)) {
-    const auto key = std::make_tuple(kernel, device, threads, smem);
+    if (context == 0) return find(kernel, threads, smem);
+    const auto key = std::make_tuple(kernel, context, threads, smem);
     std::lock_guard<std::mutex> g(ks.mu);
     auto it = ks.resident.find(key);
     if (it != ks.resident.end()) return it->second;
