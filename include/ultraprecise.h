@@ -194,7 +194,10 @@ up_status up_expr_launch_many(up_module* m, const up_column* in, int32_t n_in, c
  * per value; 2..32: the cooperative form), as chosen at compile time. */
 int32_t up_module_threads_per_value(const up_module* m);
 void up_module_release(up_module* m);
-/* Number of cached compiled kernels; clears the cache when clear != 0. */
+/* Number of cached compiled kernels; clears the cache when clear != 0, and
+ * gives back the device memory that the launches' scratch pool holds unused in
+ * the current context.  (Scratch comes from a pool of the library's own, one
+ * per context, which keeps up to 64 MB between launches.) */
 int32_t up_module_cache_size(int32_t clear);
 
 /* ------------------------------------------------- grouped aggregation */

@@ -1,5 +1,5 @@
-"""The launches' scratch pool: a device that was reset, and another thread's
-capture in progress while the pool is made."""
+"""The launches' scratch pool: a device that was reset, memory given back, and
+another thread's capture in progress while the pool is made."""
 import os
 import subprocess
 import sys
@@ -7,6 +7,9 @@ import sys
 import pytest
 
 torch = pytest.importorskip("torch")
+
+from ultraprecise_b200 import abi, runtime
+from ultraprecise_b200 import expr as E
 
 pytestmark = pytest.mark.gpu
 
@@ -54,6 +57,26 @@ def test_launches_after_a_device_reset():
     env["LD_LIBRARY_PATH"] = "/usr/local/cuda/lib64:" + env.get("LD_LIBRARY_PATH", "")
     r = subprocess.run([sys.executable, "-c", RESET], capture_output=True, text=True, timeout=300, cwd=ROOT, env=env)
     assert r.returncode == 0 and "same after the reset" in r.stdout, r.stdout + r.stderr
+
+
+def _sum_module():
+    q = runtime.compile_query([E.col(0) * E.col(1)], [(abi.UP_AGG_SUM, 0)], [E.ColType(18, 2)] * 2)
+    cols = [runtime.DeviceColumn(runtime.gen_digits(5000, 18, k), 18, 2) for k in range(2)]
+    return q, cols
+
+
+def test_unused_scratch_is_given_back():
+    groups = 600_000  # 19 MB of limb sums and more
+    q, cols = _sum_module()
+    gid = (torch.arange(5000, device="cuda") % groups).to(torch.int32)
+    outs = [torch.zeros(groups * 133, dtype=torch.uint8, device="cuda")]
+    q.launch(cols, gid, groups, outs=outs)
+    torch.cuda.synchronize()
+    held = torch.cuda.mem_get_info()[0]
+    abi.load().up_module_cache_size(1)
+    assert torch.cuda.mem_get_info()[0] >= held + (8 << 20)
+    q.launch(cols, gid, groups, outs=outs)  # and allocated anew
+    torch.cuda.synchronize()
 
 
 # a process of its own, in which no launch has made the pool yet

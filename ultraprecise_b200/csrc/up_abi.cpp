@@ -206,6 +206,13 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
     }
     return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
 }
+
+void scratch_trim() {
+    const uint64_t ctx = context_id();
+    std::lock_guard<std::mutex> g(g_pools_mu);
+    auto it = g_pools.find(ctx);
+    if (ctx != 0 && it != g_pools.end() && cudaMemPoolTrimTo(it->second, 0) != cudaSuccess) cudaGetLastError();
+}
 }  // namespace upi
 
 extern "C" {
@@ -336,7 +343,10 @@ int64_t up_module_source(const up_module* m, char* buf, int64_t cap) {
 
 void up_module_release(up_module* m) { delete m; }
 
-int32_t up_module_cache_size(int32_t clear) { return jit_cache_size(clear != 0); }
+int32_t up_module_cache_size(int32_t clear) {
+    if (clear) scratch_trim();
+    return jit_cache_size(clear != 0);
+}
 
 up_status up_expr_launch(up_module* m, const up_column* in, int32_t n_in, int64_t rows, void* out,
                          uint32_t* err_word, void* stream) {

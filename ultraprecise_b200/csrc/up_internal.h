@@ -172,9 +172,11 @@ uint64_t context_id();
 // Stream-ordered scratch from the library's own pool of the current context,
 // freed by cudaFreeAsync.  The pool keeps up to kScratchKeep bytes over a
 // synchronisation, where the default pool gives everything back to the driver
-// and the next launch allocates anew (0.4 ms and more on B200).
+// and the next launch allocates anew (0.4 ms and more on B200); scratch_trim
+// gives back what is not in use.
 constexpr uint64_t kScratchKeep = 64ull << 20;
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+void scratch_trim();
 void mkdir_if_missing(const std::string& dir);
 
 }  // namespace upi
