@@ -117,14 +117,3 @@ def test_automatic_choice_of_cooperative_path():
     assert "tpi_mul<16, 8" in prewarm.expr_source(e, cols)
     assert "up_trow" not in prewarm.expr_source(e, cols, threads_per_value=1)
     assert "tpi_div_round<8," in prewarm.expr_source(*workloads.sweep_expr(150, "div"), threads_per_value=8)
-
-
-def test_compact_bytes_refuses_what_is_no_int():
-    """Also after the same number was asked for as an int."""
-    import ctypes
-    from ultraprecise_b200 import codec
-    assert codec.compact_bytes(18) == 8
-    with pytest.raises(ctypes.ArgumentError):
-        codec.compact_bytes(18.0)
-    with pytest.raises(ValueError):
-        codec.compact_bytes(0)

@@ -16,7 +16,7 @@ import numpy as np
 from . import abi
 
 
-@lru_cache(maxsize=None, typed=True)
+@lru_cache(maxsize=None)
 def compact_bytes(p: int) -> int:
     b = abi.load().up_compact_bytes(p)
     if b < 1:
