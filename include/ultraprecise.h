@@ -341,7 +341,8 @@ int32_t up_format_width(int32_t precision, int32_t hex);
  * slot is too small).  hex != 0: the reference's output image
  * (Decimal::GetDecimal, decimal.cu:362-398: sign, 8 upper-case hex digits per
  * limb from the highest nonzero one, "(fff)" scale); hex == 0: the decimal
- * string ("-123.4500"), which parses back to the same bytes. */
+ * string ("-123.4500"), which parses back to the same bytes.  Characters past a
+ * string keep their value; the call reads and writes whole slots while it runs. */
 up_status up_format_decimal(const void* compact, int64_t rows, int32_t precision, int32_t scale, int32_t hex,
                             char* out_text, int32_t width, int32_t* out_len, void* stream);
 

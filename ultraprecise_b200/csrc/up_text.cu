@@ -436,10 +436,13 @@ __device__ __forceinline__ void decimal_chunks(u32 (&x)[N], u32 (&dig)[2 * C]) {
 // leaves in vectors.  Bound by the instructions and byte stores per
 // character; digits in local memory and byte stores to global memory waited
 // on both.  Measured on B200, 4M values of DECIMAL(38,9): 1.16 -> 0.19 ms.
+// CTAs per SM asked for (registers of 64, 102 and 255 at most): p=6 0.066 ms (0.083
+// with none asked for), p=38 0.187 (0.230), p=77 0.355 (0.357), p=200 0.477
+// (0.481); p=120 is the exception, 0.379 (0.344).
 template <int N>
-__global__ void __launch_bounds__(kTextRows, N <= 4 ? 8 : N <= 8 ? 5 : 2) k_format_staged(const u8* __restrict__ in, int64_t rows, int B, int scale,
-                                                             char* __restrict__ out, int width,
-                                                             int32_t* __restrict__ out_len) {
+__global__ void __launch_bounds__(kTextRows, N <= 4 ? 8 : N <= 8 ? 5 : 2)
+    k_format_staged(const u8* __restrict__ in, int64_t rows, int B, int scale, char* __restrict__ out, int width,
+                    int32_t* __restrict__ out_len) {
     constexpr int C = chunks_of_limbs(N), D = 8 * C;
     extern __shared__ __align__(16) u8 sm[];
     // a warp's byte stores go to rows whose slots start in different banks: four
