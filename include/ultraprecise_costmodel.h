@@ -74,7 +74,8 @@ up_status up_costmodel_set_params(up_costmodel* m, const float* params, const fl
 
 /* Threads per value with the lowest predicted time for launching the
  * expression over `rows` rows, among 1 and (when it has a cooperative form)
- * 2..32; *pred_ms (may be NULL) the predicted time. */
+ * 2..32; *pred_ms (may be NULL) the predicted time.  An ensemble leaves the
+ * width rule's choice only where its networks agree on the saving. */
 up_status up_costmodel_choose_tpv(up_costmodel* m, const up_expr_node* nodes, int32_t n_nodes, int32_t root,
                                   const up_col_type* cols, int32_t n_cols, int64_t rows, int32_t* tpv,
                                   float* pred_ms);

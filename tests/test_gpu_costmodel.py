@@ -128,3 +128,31 @@ def test_ensemble_averages_members_and_guard_keeps_the_rule():
         t, _ = ens.choose_tpv(e, cols, 1 << 20)
         assert t == costmodel.rule_tpv(e, cols), name
     ens.set_guard(0.0)
+
+
+def test_ensemble_keeps_the_rule_where_its_networks_disagree():
+    """The choice restated from every network's own predictions: the lowest mean,
+    unless the mean saving over the width rule is within the networks' spread."""
+    rng = np.random.default_rng(8)
+    nets = [costmodel.CostModel(seed=20 + k) for k in range(3)]
+    X = rng.uniform(0, 12, (256, 16)).astype(np.float32)
+    for k, net in enumerate(nets):  # networks that agree on the rows and differ on the threads per value
+        y = (0.3 * X[:, 0] + (0.1 * k - 0.1) * X[:, 1]).astype(np.float32)
+        net.train(X, y, epochs=60, batch=64, lr=3e-3, seed=k)
+    ens = costmodel.CostModel(seed=1)
+    ens.set_params(*nets[0].params())
+    ens.add_member(nets[1])
+    ens.add_member(nets[2])
+    kept = 0
+    for name, e, cols in workloads.costmodel_eval_shapes():
+        f = np.stack([costmodel.features(e, cols, t, 1 << 20)[0] for t in costmodel.TPV_CHOICES])
+        P = np.stack([n.predict(f) for n in nets]).astype(np.float64)
+        best, rule = int(np.argmin(P.mean(0))), costmodel.TPV_CHOICES.index(costmodel.rule_tpv(e, cols))
+        saving = P[:, rule] - P[:, best]
+        if abs(saving.mean() - saving.std()) < 1e-4:
+            continue
+        want = best if saving.mean() > saving.std() else rule
+        kept += want != best
+        t, _ = ens.choose_tpv(e, cols, 1 << 20)
+        assert t == costmodel.TPV_CHOICES[want], name
+    assert kept > 0

@@ -284,11 +284,14 @@ up_status predict_one(up_costmodel* m, const float* d_params, const float* norm,
     return UP_OK;
 }
 
-// The model's prediction: the mean log ms of its network and its members.
-up_status predict_locked(up_costmodel* m, const float* feats, int n, float* log_ms) {
+// The model's prediction: the mean log ms of its network and its members;
+// `each`, where given, receives every network's n predictions one after the
+// other.
+up_status predict_locked(up_costmodel* m, const float* feats, int n, float* log_ms, std::vector<float>* each = nullptr) {
     up_status st = cm_ready(m);
     if (st != UP_OK) return st;
     if ((st = predict_one(m, m->d_params, m->norm, feats, n, log_ms)) != UP_OK) return st;
+    if (each) each->assign(log_ms, log_ms + n);
     if (m->members.empty()) return UP_OK;
     std::vector<double> sum(log_ms, log_ms + n);
     std::vector<float> one(n);
@@ -299,6 +302,7 @@ up_status predict_locked(up_costmodel* m, const float* feats, int n, float* log_
                                     m->stream));
         }
         if ((st = predict_one(m, mb.d_params, mb.norm, feats, n, one.data())) != UP_OK) return st;
+        if (each) each->insert(each->end(), one.begin(), one.end());
         for (int i = 0; i < n; i++) sum[i] += one[i];
     }
     for (int i = 0; i < n; i++) log_ms[i] = (float)(sum[i] / (double)(m->members.size() + 1));
@@ -525,22 +529,39 @@ up_status up_costmodel_choose_tpv(up_costmodel* m, const up_expr_node* nodes, in
             if (st != UP_OK) return st;
         }
     float pred[6];
+    std::vector<float> each;
     {
         std::lock_guard<std::mutex> g(m->mu);
-        st = predict_locked(m, feats, nc, pred);
+        st = predict_locked(m, feats, nc, pred, &each);
     }
     if (st != UP_OK) return st;
     int best = 0;
     for (int i = 1; i < nc; i++)
         if (pred[i] < pred[best]) best = i;
-    if (m->guard > 0.0f && nc > 1) {
-        // keep the width rule's choice unless the model predicts it saves at least `guard` of the time
+    const size_t nets = each.size() / nc;
+    if ((m->guard > 0.0f || nets > 1) && nc > 1) {
         std::vector<NodeFacts> f;
         std::vector<int> topo;
         if (analyze_nodes(nodes, n_nodes, cols, n_cols, f, topo, {root}) == UP_OK) {
             const int rt = rule_threads_per_value(nodes, f, topo);
+            int rule = 0;
             for (int i = 0; i < nc; i++)
-                if (cand[i] == rt && pred[best] > pred[i] + std::log(1.0f - m->guard)) best = i;
+                if (cand[i] == rt) rule = i;
+            // keep the width rule's choice unless the model predicts it saves at
+            // least `guard` of the time, and an ensemble's networks agree on the
+            // saving: its mean (in log ms) above its standard deviation among
+            // them.  Between the widths trained on they disagree: a*b*c at p=220
+            // went to eight threads (0.81 ms, one thread 0.42) on savings of -5 to
+            // 44 %, and the held-out shapes took 5.82 ms against the rule's 5.77;
+            // 5.43 ms so, the best choices 5.41.
+            double mean = 0, sq = 0;
+            for (size_t k = 0; k < nets; k++) {
+                const double d = (double)each[k * nc + rule] - each[k * nc + best];
+                mean += d / (double)nets;
+                sq += d * d / (double)nets;
+            }
+            const bool agreed = nets < 2 || mean > std::sqrt(std::max(0.0, sq - mean * mean));
+            if (!agreed || pred[best] > pred[rule] + std::log(1.0f - m->guard)) best = rule;
         }
     }
     *tpv = cand[best];
