@@ -108,7 +108,7 @@ def test_cells_fit_the_ctas_they_are_planned_for():
         inst = [tuple(map(int, m)) for m in re.findall(r"up_query_cells_body<(\d+), (\d+), (\d+), (\d+)>\(a, sm\)", src)]
         if not inst:
             continue
-        wp = int(re.search(r"QS = \d+, WP = (\d+)", src).group(1))
+        wp = int(re.search(r"constexpr int R = \d+, WP = (\d+), NLS", src).group(1))
         tags = int(re.search(r"int\* tags = \(int\*\)\(sm \+ (\d+)\);", src).group(1))
         s, h, _, gmax = inst[0]
         assert s == h == gmax and (s == 4 or wp * s * 4 <= 40 * 1024)

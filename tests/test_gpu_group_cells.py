@@ -103,23 +103,25 @@ def test_cells_of_other_cta_sizes(threads):
 
 
 @pytest.mark.parametrize("p", [9, 18, 38, 140])
-def test_group_counts_at_the_cells_edges(p):
+@pytest.mark.parametrize("many", [False, True])
+def test_group_counts_at_the_cells_edges(p, many):
     """One group less and more than each kernel's cells hold (read from the
     generated source), by group ids and by two-byte keys whose count stays on
-    the device."""
+    the device, with so few rows that the groups past the first kernel's are
+    hashed and with enough for a cell each."""
     import re
     exprs, types = [E.col(0) * E.col(1), E.col(0)], [E.ColType(p, 2)] * 2
     src = prewarm.query_source(exprs, types, AGGS)
     slots = sorted(int(s) for s in re.findall(r"up_query_cells_body<(\d+), \d+, \d+, \d+>\(a, sm\)", src))
+    pieces = int(re.search(r"constexpr int R = \d+, WP = (\d+), NLS", src).group(1))
     assert len(slots) == 2
     q = runtime.compile_query(exprs, AGGS, types)
-    rng = random.Random(p)
+    rng = np.random.default_rng(p)
     for groups in (slots[0], slots[0] + 1, slots[1], slots[1] + 1):
-        rows = groups + 3001
+        rows = 2 ** 25 // max(pieces, 16) + 77 if many else groups + 3001
         cols = [runtime.DeviceColumn(runtime.gen_digits(rows, p, 7 + k), p, 2) for k in range(2)]
-        ids = list(range(groups)) + [int(groups * rng.random() ** 3) for _ in range(rows - groups)]
-        rng.shuffle(ids)
-        gid = torch.tensor(ids, dtype=torch.int32, device="cuda")
+        ids = np.concatenate([np.arange(groups), (groups * rng.random(rows - groups) ** 3).astype(np.int64)]).astype(np.int32)
+        gid = torch.from_numpy(rng.permutation(ids)).cuda()
         err = torch.zeros(1, dtype=torch.int32, device="cuda")
         outs = q.launch(cols, gid, groups, err=err)
         exp = oracle.query(q.built, q.aggs, [_raw(c.data) for c in cols], _raw(gid), rows, groups, threads=8)

@@ -516,7 +516,7 @@ size_t query_scratch_bytes(const GeneratedModule& g, int32_t n_groups) {
 }
 
 size_t query_scratch_bytes_max(const GeneratedModule& g, int32_t n_groups) {
-    const size_t limb = g.q_gs > 0 && n_groups > g.q_gs
+    const size_t limb = g.q_gs > 0 && n_groups > g.q_gs_h
                             ? query_scratch_bytes(g, g.q_gs) + 32u + (size_t)n_groups * g.q_limb_words * 8u
                             : 0u;
     return std::max(limb, query_scratch_bytes(g, n_groups));
@@ -552,10 +552,14 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
     // out small enough for the cells, whose accumulators it keeps.  Where they
     // do not fit the caller's scratch or limit, or the device, the accumulators
     // alone do, as for 2^31 rows.
-    bool limbs = contig && g.q_staged && g.q_gs > 0 && n_groups > g.q_gs && rows < ((int64_t)1 << 31);
+    const bool keys_aligned = keys ? aligned16(keys->key0) && (keys->mode != 2 || aligned16(keys->key1)) : aligned16(group_ids);
+    const bool direct = vec_ok && keys_aligned && rows >= kDirectWork / std::max(g.q_pieces, 16);
+    int32_t cell_groups = direct ? g.q_gs : g.q_gs_h;
+    bool limbs = contig && g.q_staged && g.q_gs > 0 && n_groups > cell_groups && rows < ((int64_t)1 << 31);
     size_t acc_bytes = 0, limb_off = 0, need = 0;
     auto size_scratch = [&]() {
-        const int32_t acc_groups = limbs ? (device_count ? g.q_gs : 0) : n_groups;
+        if (!limbs) cell_groups = g.q_gs;
+        const int32_t acc_groups = limbs ? (device_count ? cell_groups : 0) : n_groups;
         acc_bytes = (((size_t)acc_groups * accw * 4u) + 15u) & ~(size_t)15u;
         limb_off = (query_scratch_bytes(g, acc_groups) + 31u) & ~(size_t)31u;
         need = limbs ? limb_off + (size_t)n_groups * g.q_limb_words * 8u : query_scratch_bytes(g, n_groups);
@@ -590,13 +594,12 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
     a.err = err_word;
     a.n_groups = device_count ? -n_groups : n_groups;
     a.vec_ok = vec_ok ? 1 : 0;
-    bool keys_aligned = aligned16(group_ids);
+    a.cell_groups = cell_groups;
     if (keys) {
         a.key0 = keys->key0;
         a.key1 = keys->key1;
         a.key_table = keys->table;
         a.key_mode = keys->mode;
-        keys_aligned = aligned16(keys->key0) && (keys->mode != 2 || aligned16(keys->key1));
     }
     void* args[1] = {&a};
     if (e == cudaSuccess && rows > 0) {
@@ -609,8 +612,8 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
             const char* lo_name = keys ? "up_query_tile_rk_lo" : "up_query_tile_r_lo";
             const char* name = reg_lo                                               ? lo_name
                                : reg                                                ? reg_name
-                               : n_groups > g.q_gs_h && n_groups <= g.q_gs ? "up_query_tile_d"
-                               : (n_groups <= g.q_gs || a.lacc)             ? "up_query_tile_h"
+                               : n_groups > g.q_gs_h && n_groups <= cell_groups ? "up_query_tile_d"
+                               : (n_groups <= cell_groups || a.lacc)            ? "up_query_tile_h"
                                                                                     : "up_query_tile_g";
             a.vec_ok = (vec_ok && keys_aligned) ? 1 : 0;
             auto launch_tile = [&](const char* kname) -> cudaError_t {
@@ -636,8 +639,8 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
                 if (g.q_gr_lo > 0) e = launch_tile(lo_name);
                 if (e == cudaSuccess && g.q_gr > 0 && n_groups > g.q_gr_lo) e = launch_tile(reg_name);
                 if (e == cudaSuccess && (g.q_gr == 0 || n_groups > g.q_gr)) e = launch_tile("up_query_tile_h");
-                if (e == cudaSuccess && g.q_gs > g.q_gs_h && n_groups > g.q_gs_h) e = launch_tile("up_query_tile_d");
-                if (e == cudaSuccess && n_groups > g.q_gs && !a.lacc) e = launch_tile("up_query_tile_g");
+                if (e == cudaSuccess && cell_groups > g.q_gs_h && n_groups > g.q_gs_h) e = launch_tile("up_query_tile_d");
+                if (e == cudaSuccess && n_groups > cell_groups && !a.lacc) e = launch_tile("up_query_tile_g");
             } else {
                 e = launch_tile(name);
             }

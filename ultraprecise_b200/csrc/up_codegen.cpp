@@ -1529,12 +1529,12 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         int S = 2048;
         while (S > 4 && WP * S * 4 > kCellBytes) S /= 2;
         // More groups than S, up to S2: a kernel with one cell per group and two
-        // CTAs per SM.  S2 is whole warps of slots; where that is no more than S
-        // there is no such kernel.  Measured on B200, 16M rows of SUM(a*b), AVG(a):
-        // at p=38 (S 256, S2 960) 400 groups 1.33 ms hashed, 0.39 ms so; at p=18
-        // (512, 1824) 1000 groups 0.83 and 0.25 ms.  For fewer groups _h is the
-        // faster one: its smaller CTAs are more per SM (p=18, 400 groups 0.17 ms;
-        // with three CTAs of 75 KB 0.20 ms).
+        // CTAs per SM, for launches large enough (kDirectWork).  S2 is whole
+        // warps of slots; where that is no more than S there is no such kernel.
+        // Measured on B200, 16M rows of SUM(a*b), AVG(a): at p=38 (S 256, S2 960) 400
+        // groups 1.33 ms hashed, 0.39 ms so; at p=18 (512, 1824) 1000 groups 0.83
+        // and 0.25 ms.  For fewer groups _h is the faster one: its smaller CTAs are
+        // more per SM (p=18, 400 groups 0.17 ms; with three CTAs of 75 KB 0.20 ms).
         const int off_tag = 2 * sh.bytes;
         int S2 = std::min(kDirectSlots, (kTwoCtaSmem - off_tag - 32) / (4 * WP)) / 32 * 32;
         if (S2 <= S) S2 = S;
@@ -1543,6 +1543,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         auto cells_smem = [&](int slots, int tags) { return off_tag + tags * 4 + (WP * slots * 4 + 15) / 16 * 16 + 16; };
         out.q_gs_h = S;
         out.q_gs = S2;
+        out.q_pieces = WP;
         out.q_limb_words = NLS;
         out.q_smem_h = cells_smem(S, S);
         out.q_smem_d = cells_smem(S2, 0);
@@ -1647,14 +1648,15 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         // SUM(a*b), AVG(a), COUNT at p=18 over 100 000 groups of Zipf(1.1)
         // sizes: 12.4 ms with global carry chains, 0.61 ms this way.
         // S: cells, one or more per group for GMIN < groups <= GMAX; H: slots of the
-        // hash for more than QS groups (0: none).
+        // hash for more than a.cell_groups groups (0: none).
         src << "template <int S, int H, int GMIN, int GMAX>\nUP_DI void up_query_cells_body(const UpQArgs& a, u8* sm) {\n";
-        src << "    constexpr int R = " << R << ", QS = " << S2 << ", WP = " << WP << ", NLS = " << NLS << ";\n";
+        src << "    constexpr int R = " << R << ", WP = " << WP << ", NLS = " << NLS << ";\n";
         src << "    int* tags = (int*)(sm + " << off_tag << ");\n    int* cells = tags + H;\n";
         src << "    u64* bar = (u64*)(sm + " << off_tag << " + H * 4 + (WP * S * 4 + 15) / 16 * 16);\n";
         src << "    const int ng = q_groups(a);\n";
         src << "    if (ng < 0) { if (threadIdx.x == 0 && blockIdx.x == 0 && a.err) atomicOr(a.err, ERR_DOMAIN); return; }\n";
-        src << "    const bool hashed = H > 0 && ng > QS;\n    if (hashed ? !a.lacc : ng <= GMIN || ng > GMAX) return;\n";
+        src << "    const bool hashed = H > 0 && ng > a.cell_groups;\n"
+               "    if (hashed ? !a.lacc : ng <= GMIN || ng > GMAX || ng > a.cell_groups) return;\n";
         src << "    int rep = 1;  // replicas per group: lanes of a warp rarely meet on a cell\n";
         src << "    if (!hashed)\n        for (rep = 32; ng * rep > S;) rep >>= 1;\n";
         src << "    const int lane = threadIdx.x & 31;\n";
@@ -1714,7 +1716,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         src << "    constexpr int R = " << R << ";\n    u64* bar = (u64*)(sm + " << 2 * sh.bytes << ");\n";
         src << "    const int ng = q_groups(a);\n";
         src << "    if (ng < 0) { if (threadIdx.x == 0 && blockIdx.x == 0 && a.err) atomicOr(a.err, ERR_DOMAIN); return; }\n";
-        src << "    if (ng <= " << S2 << " || a.lacc) return;\n";
+        src << "    if (ng <= a.cell_groups || a.lacc) return;\n";
         src << "    const i64 ntiles = (a.rows + R - 1) / R;\n";
         src << "    const i64 nfull = a.vec_ok ? a.rows / R : 0;  // tiles moved by bulk copies\n";
         src << "    u32 err = 0u;\n" << tile_pipeline_open(sh);
@@ -1889,7 +1891,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
     src << "    const i64 g = g0 + ((int)threadIdx.x < nb ? (int)threadIdx.x : 0);  // the CTA's other threads repeat its first group\n";
     src << "    u8* img = imgs + threadIdx.x * " << UP_AGG_DECIMAL_BYTES << ";\n";
     if (out.q_gs > 0) {  // limb sums or accumulators, by the rule of the tile kernels
-        src << "    const bool hashed = a.lacc && q_groups(a) > " << out.q_gs << ";\n";
+        src << "    const bool hashed = a.lacc && q_groups(a) > a.cell_groups;\n";
         src << "    const i64* lac = a.lacc + (i64)g * " << out.q_limb_words << ";\n";
         int nlt = 0;
         for (int i = 0; i < NR; i++) nlt += f[acc_root[i]].limbs;

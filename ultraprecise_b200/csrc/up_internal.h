@@ -80,6 +80,15 @@ int coop_width_of(const up_expr_node* nodes, int n_nodes, int root, const up_col
 
 // ------------------------------------------------------------ code generation
 constexpr int kFinGroups = 128;  // groups per CTA of up_query_fin
+// Rows times pieces (at least 16) from which up_query_tile_d is launched: its
+// 113 KB of cells per CTA are cleared and folded whatever the rows.  Measured on
+// B200, hashed against one cell per group, uniform and Zipf(1.1) ids: p=9 (7
+// pieces), 3000 groups, 1M rows 49 / 49 and 39 / 44 us, 2M 84 / 59 and 57 / 54; p=38
+// (25), 500 groups, 500K rows 66 / 62 and 58 / 56, 2M 210 / 91 and 109 / 97; 100K rows
+// of either 13-25 / 33-37 us.  Not for columns off 16-byte boundaries either,
+// which are copied a byte at a time: two CTAs per SM wait for that (4M rows at
+// p=38, 400 groups 0.48 / 1.03 ms).
+constexpr int64_t kDirectWork = 1ll << 25;
 struct GeneratedModule {
     std::string source;
     std::vector<std::string> kernels;
@@ -100,6 +109,7 @@ struct GeneratedModule {
     int q_gr_lo = 0;              // up_query_tile_r_lo handles n_groups <= q_gr_lo (0: no such kernel)
     int q_gs = 0;                 // groups with a cell each: direct for n_groups <= q_gs, else hashed
     int q_gs_h = 0;               // of them up_query_tile_h's (which also hashes); up_query_tile_d takes the rest
+    int q_pieces = 0;             // cells of one group
     int q_limb_words = 0;         // 64-bit words of one group's limb sums (hashed launches)
     int q_smem = 0;               // dynamic shared memory of up_query_tile_g
     int q_smem_h = 0;             // of up_query_tile_h

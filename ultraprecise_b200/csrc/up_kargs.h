@@ -40,7 +40,8 @@ struct UpArgs {
 // (2), or key0[2r] << 8 | key0[2r+1] (3).  n_groups < 0: the count is read
 // from the key table on the device, -n_groups being the capacity.  lacc: the
 // limb sums of a launch whose groups outnumber its shared-memory cells (NULL:
-// its accumulators are in acc like the others').
+// its accumulators are in acc like the others').  cell_groups: up to how many
+// groups have a cell each; more are hashed.
 struct UpQArgs {
     UpKCol col[UP_MAX_COLS];
     unsigned char* out[UP_MAX_AGGS];
@@ -56,6 +57,7 @@ struct UpQArgs {
     const int* key_table;
     long long* lacc;
     int key_mode;
+    int cell_groups;
 };
 
 // Batch modules: one task of the work queue, and the band kernels' arguments.
