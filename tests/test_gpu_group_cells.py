@@ -132,3 +132,41 @@ def test_group_counts_at_the_cells_edges(p, many):
         assert int(err.item()) == 0
         for k, e in enumerate(exp):
             assert _raw(outs[k]) == e and _raw(got[k])[:len(e)] == e, (groups, k)
+
+
+@pytest.mark.parametrize("p", [5, 15, 38])
+@pytest.mark.parametrize("rows", [1, 255, 2047, 30_001])
+def test_columns_off_16_byte_boundaries(p, rows):
+    """Columns, group ids and keys that bulk copies cannot take: each kernel's
+    tiles copied in bytes, several per thread and the rest one by one."""
+    a, b = E.col(0), E.col(1)
+    q = runtime.compile_query([a * b, a - b], AGGS, [E.ColType(p, 2)] * 2)
+    raws = [runtime.gen_digits(rows, p, 7 + k) for k in range(2)]
+    rng = np.random.default_rng(rows)
+
+    def off(t, shift):
+        t = t.contiguous().view(torch.uint8)
+        buf = torch.zeros(t.numel() + 16, dtype=torch.uint8, device="cuda")
+        buf[shift:shift + t.numel()] = t
+        return buf[shift:shift + t.numel()]
+
+    cols = [runtime.DeviceColumn(off(t, 1 + 2 * k), p, 2) for k, t in enumerate(raws)]
+    for groups in (3, 40, 3000):
+        ids = rng.integers(0, groups, rows).astype(np.int32)
+        gid = off(torch.from_numpy(ids).cuda(), 4).view(torch.int32)
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        outs = q.launch(cols, gid, groups, err=err)
+        exp = oracle.query(q.built, q.aggs, [_raw(t) for t in raws], ids.tobytes(), rows, groups, threads=8)
+        assert int(err.item()) == 0
+        for k, e in enumerate(exp):
+            assert _raw(outs[k]) == e, (groups, k)
+        if groups == 40:
+            keys = [off(torch.from_numpy((ids % 5).astype(np.uint8)).cuda(), 3)]
+            table = torch.zeros(abi.UP_KEY_TABLE_ENTRIES, dtype=torch.int32, device="cuda")
+            runtime.group_table_from_keys_async(keys, [1], table)
+            kid, n, _ = runtime.group_ids_from_keys(keys, [1])
+            got = q.launch_keys_async(cols, keys, [1], table, 8, err=err, rows=rows)
+            exp = oracle.query(q.built, q.aggs, [_raw(t) for t in raws], _raw(kid), rows, n, threads=8)
+            assert int(err.item()) == 0
+            for k, e in enumerate(exp):
+                assert _raw(got[k])[:len(e)] == e, k

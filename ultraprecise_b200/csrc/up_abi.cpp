@@ -604,10 +604,11 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
     void* args[1] = {&a};
     if (e == cudaSuccess && rows > 0) {
         if (contig && g.q_staged) {
-            // staged tiles; accumulators in registers, shared memory or global
-            // memory by group count
-            const bool reg = g.q_gr > 0 && n_groups <= g.q_gr;
-            const bool reg_lo = g.q_gr_lo > 0 && n_groups <= g.q_gr_lo;
+            // staged tiles; accumulators in registers (aligned columns), shared
+            // memory or global memory by group count
+            const bool aligned = vec_ok && keys_aligned;
+            const bool reg = aligned && g.q_gr > 0 && n_groups <= g.q_gr;
+            const bool reg_lo = aligned && g.q_gr_lo > 0 && n_groups <= g.q_gr_lo;
             const char* reg_name = keys ? "up_query_tile_rk" : "up_query_tile_r";
             const char* lo_name = keys ? "up_query_tile_rk_lo" : "up_query_tile_r_lo";
             const char* name = reg_lo                                               ? lo_name
@@ -615,7 +616,7 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
                                : n_groups > g.q_gs_h && n_groups <= cell_groups ? "up_query_tile_d"
                                : (n_groups <= cell_groups || a.lacc)            ? "up_query_tile_h"
                                                                                     : "up_query_tile_g";
-            a.vec_ok = (vec_ok && keys_aligned) ? 1 : 0;
+            a.vec_ok = aligned ? 1 : 0;
             auto launch_tile = [&](const char* kname) -> cudaError_t {
                 void* k = jit_kernel(*m->jm.ks, kname);
                 const char mode = kname[14];  // up_query_tile_<mode>
@@ -636,9 +637,9 @@ up_status query_launch_ex(up_module* m, const up_column* in, int32_t n_in, int64
             if (device_count) {
                 // the mode follows the count on the device: every applicable
                 // mode kernel is launched and all but one return at once
-                if (g.q_gr_lo > 0) e = launch_tile(lo_name);
-                if (e == cudaSuccess && g.q_gr > 0 && n_groups > g.q_gr_lo) e = launch_tile(reg_name);
-                if (e == cudaSuccess && (g.q_gr == 0 || n_groups > g.q_gr)) e = launch_tile("up_query_tile_h");
+                if (aligned && g.q_gr_lo > 0) e = launch_tile(lo_name);
+                if (e == cudaSuccess && aligned && g.q_gr > 0 && n_groups > g.q_gr_lo) e = launch_tile(reg_name);
+                if (e == cudaSuccess && (!aligned || g.q_gr == 0 || n_groups > g.q_gr)) e = launch_tile("up_query_tile_h");
                 if (e == cudaSuccess && cell_groups > g.q_gs_h && n_groups > g.q_gs_h) e = launch_tile("up_query_tile_d");
                 if (e == cudaSuccess && n_groups > cell_groups && !a.lacc) e = launch_tile("up_query_tile_g");
             } else {

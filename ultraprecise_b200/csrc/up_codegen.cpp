@@ -235,6 +235,26 @@ UP_DI int q_groups(const UpQArgs& a) {
     const int n = *(volatile const int*)(a.key_table + 131072);
     return (n >= 0 && n <= -a.n_groups) ? n : -1;
 }
+// tile_copy_in with eight bytes of a thread in flight where it goes by bytes:
+// columns off 16-byte boundaries, which the cells' kernels take at any number of
+// groups (one byte at a time waits for the memory each time: 4M rows of SUM(a*b),
+// AVG(a) at p=38 in four groups 0.97 ms in the register kernels, 0.16 ms so)
+UP_DI void q_copy_in(u8* __restrict__ dst, const u8* __restrict__ src, int n, bool vec_ok) {
+    if (vec_ok && (n & 15) == 0) {
+        tile_copy_vec((uint4*)dst, (const uint4*)src, n >> 4);
+        return;
+    }
+    const int T = blockDim.x;
+    int i = threadIdx.x;
+    for (; i + 7 * T < n; i += 8 * T) {
+        u8 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = src[i + k * T];
+#pragma unroll
+        for (int k = 0; k < 8; k++) dst[i + k * T] = v[k];
+    }
+    for (; i < n; i += T) dst[i] = src[i];
+}
 // the keys (or group ids) of rows 4q .. 4q+3 of a staged tile of R rows
 template <int KEYS, int R>
 UP_DI void q_quad_keys(const UpQArgs& a, const u8* t, int q, u32 (&k)[4]) {
@@ -1552,8 +1572,10 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         // The tile loop of every staged kernel: the next tile's bulk copies are
         // issued before the current tile is waited for; opens the loop body,
         // with tile t's rows [row0, row0 + nr) at `in` and their groups at `tg`.
-        // `stop`: the statement that leaves the loop after a timeout.
-        auto tile_pipeline_open = [&](const Stage& g, const char* stop = "if (__syncthreads_or(timed_out)) break;") {
+        // `copy` moves the tiles that bulk copies do not; `stop` is the statement that
+        // leaves the loop after a timeout.
+        auto tile_pipeline_open = [&](const Stage& g, const std::string& copy = "q_copy_in",
+                                      const char* stop = "if (__syncthreads_or(timed_out)) break;") {
             std::ostringstream src;
             const int R = g.rows;
             int tile_in_bytes = 0;
@@ -1595,15 +1617,15 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
             for (size_t i = 0; i < used.size(); i++) {
                 int c = used[i];
                 int B = compact_bytes(cols[c].precision);
-                src << "            tile_copy_in(in + " << g.off[i] << ", a.col[" << c << "].data + row0 * " << B << ", nr * "
+                src << "            " << copy << "(in + " << g.off[i] << ", a.col[" << c << "].data + row0 * " << B << ", nr * "
                     << B << ", a.vec_ok != 0);\n";
             }
-            src << "            if (a.key_mode == 0) tile_copy_in(in + " << g.gid
+            src << "            if (a.key_mode == 0) " << copy << "(in + " << g.gid
                 << ", (const u8*)(a.gid + row0), nr * 4, a.vec_ok != 0);\n";
-            src << "            else if (a.key_mode == 3) tile_copy_in(in + " << g.gid
+            src << "            else if (a.key_mode == 3) " << copy << "(in + " << g.gid
                 << ", a.key0 + row0 * 2, nr * 2, a.vec_ok != 0);\n";
-            src << "            else {\n                tile_copy_in(in + " << g.gid << ", a.key0 + row0, nr, a.vec_ok != 0);\n";
-            src << "                if (a.key_mode == 2) tile_copy_in(in + " << g.gid + R
+            src << "            else {\n                " << copy << "(in + " << g.gid << ", a.key0 + row0, nr, a.vec_ok != 0);\n";
+            src << "                if (a.key_mode == 2) " << copy << "(in + " << g.gid + R
                 << ", a.key1 + row0, nr, a.vec_ok != 0);\n            }\n";
             src << "            __syncthreads();\n";
             src << "        }\n";
@@ -1656,7 +1678,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
         src << "    const int ng = q_groups(a);\n";
         src << "    if (ng < 0) { if (threadIdx.x == 0 && blockIdx.x == 0 && a.err) atomicOr(a.err, ERR_DOMAIN); return; }\n";
         src << "    const bool hashed = H > 0 && ng > a.cell_groups;\n"
-               "    if (hashed ? !a.lacc : ng <= GMIN || ng > GMAX || ng > a.cell_groups) return;\n";
+               "    if (hashed ? !a.lacc : ng <= (H > 0 && !a.vec_ok ? 0 : GMIN) || ng > GMAX || ng > a.cell_groups) return;\n";
         src << "    int rep = 1;  // replicas per group: lanes of a warp rarely meet on a cell\n";
         src << "    if (!hashed)\n        for (rep = 32; ng * rep > S;) rep >>= 1;\n";
         src << "    const int lane = threadIdx.x & 31;\n";
@@ -1827,7 +1849,7 @@ up_status generate_query_module(const up_expr_node* nodes, int n_nodes, const up
             // groups: 0.49 -> 0.40 ms (0.43 with 128-bit sums in registers before
             // the narrow evaluation); over money rows 0.226 -> 0.222 ms.
             src << "    bool general = false;\n"
-                << tile_pipeline_open(sr, "const bool ask = __syncthreads_or(timed_out || general);\n"
+                << tile_pipeline_open(sr, "tile_copy_in", "const bool ask = __syncthreads_or(timed_out || general);\n"
                                           "        if (ask && __syncthreads_or(timed_out)) break;\n"
                                           "        const bool mostly = ask && (k & 7) != 0;\n        general = false;");
             src << "        if (mostly) {\n            wide = general = true;\n";
